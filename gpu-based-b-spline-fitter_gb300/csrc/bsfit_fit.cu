@@ -1,5 +1,6 @@
 // Host side of the FP32 fitter kernels (bsfit_fit_kernels.cuh): launch shapes,
 // the plain, batched and evaluation launches, and the FP32 peak probe.
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <mutex>
@@ -96,7 +97,7 @@ struct LaunchChoice {
   int per_warp, dev, force, wpb, bps, sms;
 };
 std::mutex g_choice_mu;
-constexpr int kMaxChoices = 128;
+constexpr int kMaxChoices = 256;
 LaunchChoice g_choices[kMaxChoices];
 int g_nchoices = 0;
 struct RaisedKernel {
@@ -106,6 +107,15 @@ struct RaisedKernel {
 RaisedKernel g_raised[128];
 int g_nraised = 0;
 }  // namespace
+
+cudaError_t sm_count(int dev, int* sms) {
+  static std::atomic<int> known[64];  // per device; 0: not asked yet
+  if (dev >= 0 && dev < 64 && (*sms = known[dev].load(std::memory_order_relaxed)) > 0)
+    return cudaSuccess;
+  const cudaError_t e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) known[dev].store(*sms, std::memory_order_relaxed);
+  return e;
+}
 
 cudaError_t pick_launch(const void* kern, int per_warp, int* wpb, int* bps, int* sms) {
   return pick_launch_wpb(kern, per_warp, 0, wpb, bps, sms);
@@ -138,7 +148,7 @@ cudaError_t pick_launch_wpb(const void* kern, int per_warp, int force_wpb, int* 
     if (g_nraised < 128) g_raised[g_nraised++] = RaisedKernel{kern, dev};
   }
   int best = -1, bw = 4, bb = 0;
-  for (int cand = 4; cand >= 1; cand >>= 1) {
+  for (int cand = force_wpb ? force_wpb : 4; cand >= 1; cand >>= 1) {
     if (force_wpb && cand != force_wpb) continue;
     const int sm = per_warp * cand;
     if (sm > optin) continue;
@@ -376,6 +386,11 @@ cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream) {
     // double-float kernels: plain EMCCD fits of fit types 6, 7, 8, one start
     if (a.var || a.n_starts > 1 || a.trace || a.m.fittype == kFit4Pi) return cudaErrorInvalidValue;
     return launch_fitdd(a, stream);
+  }
+  {
+    bool taken = false;
+    const cudaError_t et = launch_team(a, &taken, stream);
+    if (taken || et != cudaSuccess) return et;
   }
   const int mode = a.m.fittype;
   const bool var = a.var != nullptr;

@@ -276,20 +276,21 @@ __device__ __forceinline__ int hidx(int l, int m) {
   return l * NV - (l * (l - 1)) / 2 + (m - l);
 }
 
-// floor(a / b) for 0 <= a <= 64 and 1 <= b <= 64 without an integer division:
+// floor(a / b) for 0 <= a <= 1024 and 1 <= b <= 64 without an integer division:
 // q = trunc(a * r + 2^-10) with r the approximate reciprocal of b (relative
-// error at most 2^-21). When a / b is an integer k <= 64, a * r >= k - 2^-15
-// and the 2^-10 lifts it above k; otherwise a / b <= k + 1 - 1/b with
-// 1/b >= 2^-6, so a * r + 2^-10 < k + 1 - 2^-6 + 2^-15 + 2^-10 < k + 1. The
-// window and ROI widths (at most 55) and lane counts stay in that domain.
+// error at most 2^-21). When a / b is an integer k <= 1024, a * r >= k - 2^-11
+// and the 2^-10 lifts it above k (the sum's own rounding is at most 2^-14);
+// otherwise a / b <= k + 1 - 1/b with 1/b >= 2^-6, so a * r + 2^-10 <
+// k + 1 - 2^-6 + 2^-11 + 2^-10 + 2^-14 < k + 1. The window and ROI widths (at
+// most 55) and the thread counts of a warp or a block stay in that domain.
 __device__ __forceinline__ int small_div(int a, int b) {
   const float r = __fdividef(1.0f, (float)b);
   return __float2int_rz(fmaf((float)a, r, 0.0009765625f));
 }
 
 // Row/column of item t of a row-major (rows x w) grid for a lane that starts at
-// t = lane and advances by `step` (32, or 16 for a half-warp's lanes): avoids a
-// runtime integer division per item.
+// t = lane and advances by `step` (32, 16 for a half-warp's lanes, or a block's
+// threads): avoids a runtime integer division per item.
 struct Stride2D {
   int r, c, dr, dc, w;
   __device__ __forceinline__ Stride2D(int lane, int w_, int step = 32) : w(w_) {
@@ -331,22 +332,40 @@ __device__ __forceinline__ float wrap_phase(float w, int nw) {
 // l sums those pixels into (err, acc) and pixels l + 16, l + 48, ... (the
 // sequence of warp lane l + 16) into (err2, acc2), so the reductions that
 // follow can form the same sums as the whole warp's.
-template <int MODE, int KP, bool VAR, int STG = 0, int LW = 32>
+//
+// TW > 0: TW warps of a block work on the ROI's channel (bsfit_team.cuh). The
+// stages are shared by their threads (tt: this one's index among them) and
+// separated by block barriers, every warp keeps its own knots and weights in kws (no barrier for them), and stage C
+// writes each pixel's terms to rec (field f of pixel p at rec[f * L.s2p + p]:
+// the deviance or log-likelihood term, t1, t2, then the NV derivatives) instead
+// of summing them; the team then forms the same sums from the records.
+template <int MODE, int KP, bool VAR, int STG = 0, int LW = 32, int TW = 0>
 __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout& L, float* ws,
                                              const float* data, int lane, const float* th,
                                              bool dup45, bool FISHER, FPair& err,
                                              float (&acc)[KP], FPair& err2, float (&acc2)[KP],
-                                             unsigned gm = kFull, bool maps_ready = false) {
+                                             unsigned gm = kFull, bool maps_ready = false,
+                                             float* kws = nullptr, float* rec = nullptr,
+                                             int tt = 0, const Stride2D* walk = nullptr) {
   static_assert(LW == 32 || (LW == 16 && MODE == 6 && !VAR && STG == 0),
                 "half-warp ROIs: the 3D EMCCD model only");
+  static_assert(TW == 0 || (LW == 32 && STG == 0), "a team is made of whole warps");
   using TR = ModeTraits<MODE>;
   constexpr int D = TR::D;
   constexpr int NV = TR::NV;
   const int s = L.s;
   const ModelDev& m = a.m;
-  int* kxs = reinterpret_cast<int*>(ws + L.off_kx());
-  int* kys = reinterpret_cast<int*>(ws + L.off_ky());
-  float* w = ws + L.off_w();
+  float* kb = (TW > 0) ? kws : ws;
+  int* kxs = reinterpret_cast<int*>(kb + L.off_kx());
+  int* kys = reinterpret_cast<int*>(kb + L.off_ky());
+  float* w = kb + L.off_w();
+  // this thread's first item and the item stride of the shared stages
+  const int t_first = (TW > 0) ? tt : lane;
+  constexpr int TS = (TW > 0) ? 32 * TW : LW;
+  auto stage_sync = [] {
+    if constexpr (TW > 0) __syncthreads();
+    else __syncwarp();
+  };
   float* A = ws + L.off_a();  // A[xr * AS + map * wp + yr]
   float* G = ws + L.off_g();  // G[(xr * s + py) * GP + map]
   const int wp = L.wp;
@@ -363,39 +382,35 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
   const float wc = (D >= 4) ? th[5] : 0.0f;
   const float uc = (D >= 5) ? th[6] : 0.0f;
 
-  for (int j = lane; j < s; j += LW) {
-    kxs[j] = knot_index((xc + (float)j) + off, m.n[1]);
-    kys[j] = knot_index((yc + (float)j) + off, m.n[0]);
-  }
-  // Fractional parts (Y, X, Z, W) and the 1-D weights, one per lane.
-  {
-    float fr[5];
-    fr[0] = yc - floorf(yc);
-    fr[1] = xc - floorf(xc);
-    fr[2] = zc - floorf(zc);
-    fr[3] = wc - floorf(wc);
-    fr[4] = uc - floorf(uc);
-    // 7 weights per axis: 35 for the 5D model, more than one per lane.
-    for (int k = lane; k < 7 * D; k += LW) {
-      const int ax = k / 7;
-      w[ax * 8 + (k - ax * 7)] = axis_weight(fr[ax], k - ax * 7);
-    }
-  }
-  __syncwarp();
+  // Knots of the pixel columns and rows (each lane keeps to its own until the
+  // window is known) and their range; the fractional parts (Y, X, Z, W, U) and
+  // the 1-D weights, one per lane: 35 for the 5D model, more than one per lane.
   int kxmin, kxmax, kymin, kymax;
   {
     int a0 = INT_MAX, a1 = INT_MIN, b0 = INT_MAX, b1 = INT_MIN;
     for (int j = lane; j < s; j += LW) {
-      a0 = min(a0, kxs[j]);
-      a1 = max(a1, kxs[j]);
-      b0 = min(b0, kys[j]);
-      b1 = max(b1, kys[j]);
+      const int kx = knot_index((xc + (float)j) + off, m.n[1]);
+      const int ky = knot_index((yc + (float)j) + off, m.n[0]);
+      kxs[j] = kx;
+      kys[j] = ky;
+      a0 = min(a0, kx);
+      a1 = max(a1, kx);
+      b0 = min(b0, ky);
+      b1 = max(b1, ky);
+    }
+    for (int k = lane; k < 7 * D; k += LW) {
+      const int ax = (k * 37) >> 8;  // k / 7 for k < 35
+      float p = ax == 0 ? yc : ax == 1 ? xc : zc;
+      if (D >= 4 && ax == 3) p = wc;
+      if (D >= 5 && ax == 4) p = uc;
+      w[ax * 8 + (k - ax * 7)] = axis_weight(p - floorf(p), k - ax * 7);
     }
     kxmin = __reduce_min_sync(gm, a0);
     kxmax = __reduce_max_sync(gm, a1);
     kymin = __reduce_min_sync(gm, b0);
     kymax = __reduce_max_sync(gm, b1);
   }
+  __syncwarp();
   // Window of lateral nodes [k - 1, k + 2] over all pixels. Its extent is at
   // most s + 4 (the per-pixel knots grow by one per pixel, plus one for
   // rounding); the caps keep every shared-memory access inside the warp's maps.
@@ -403,7 +418,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
   const int yb = kymin - 1, wy = min(kymax - kymin + 4, wp);
   // Per pixel row: the window offset of its first Y node (clamped so the four
   // reads stay in the window); per pixel column: that of its first X node,
-  // times the G column stride. Written over the knots by the lane that read
+  // times the G column stride. Written over the knots by the lane that wrote
   // them; stages B and C read them after the synchronisation that ends stage A.
   for (int j = lane; j < s; j += LW) {
     kxs[j] = min(max(kxs[j] - 1 - xb, 0), wx - 4) * GS;
@@ -433,8 +448,8 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       const float* b2 = b1 + sz_;
       const float* b3 = b2 + sz_;
       const int st1 = (int)m.st[1];
-      Stride2D ix(lane, wy, LW);
-      for (int t = lane; t < nodes; t += LW, ix.next()) {
+      Stride2D ix(t_first, wy, TS);
+      for (int t = t_first; t < nodes; t += TS, ix.next()) {
         const int xr = ix.r, yr = ix.c;
         const int lat = (xb + xr) * st1 + (yb + yr);
         float c0 = __ldg(b0 + lat), c1 = __ldg(b1 + lat), c2 = __ldg(b2 + lat), c3 = __ldg(b3 + lat);
@@ -451,7 +466,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       // lateral offsets from one base per entry set (lateral planes hold fewer
       // than 2^29 elements).
       const int st1 = (int)m.st[1];
-      Stride2D ix(lane, wy);
+      Stride2D ix(t_first, wy, TS);
       const float2 BZ0 = bc2(bz0), BZ1 = bc2(bz1), BZ2 = bc2(bz2), BZ3 = bc2(bz3);
       const float2 DZ0 = bc2(dz0), DZ1 = bc2(dz1), DZ2 = bc2(dz2);
       // 4Pi: the four z planes of layer kw - 1 + iw at q4 + iw * zq_w; fit
@@ -460,7 +475,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       const float4* q4 = m.zq + (int64_t)(kw - 1) * m.zq_w + (int64_t)(kz - 1) * m.zq_kz;
       const float4* qp[2] = {q4, q4 + 2 * m.zq_w};
       const int plane = (int)m.st[2];
-      for (int t = lane; t < nodes; t += 32, ix.next()) {
+      for (int t = t_first; t < nodes; t += TS, ix.next()) {
         const int xr = ix.r, yr = ix.c;
         const int o0 = (xb + xr) * st1 + (yb + yr);
         // z contraction of the four w layers: two layers per packed operation
@@ -665,8 +680,8 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       // part's four z planes from the gather table (32-bit lateral offsets)
       const int st1 = (int)m.st[1];
       const float4* q3 = m.zq + (int64_t)(kz - 1) * m.zq_kz;
-      Stride2D ix(lane, wy);
-      for (int t = lane; t < nodes; t += 32, ix.next()) {
+      Stride2D ix(t_first, wy, TS);
+      for (int t = t_first; t < nodes; t += TS, ix.next()) {
         const int xr = ix.r, yr = ix.c;
         const int o0 = (xb + xr) * st1 + (yb + yr);
         const float* p = base + o0;
@@ -743,7 +758,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       }
     }
   }
-  __syncwarp();
+  stage_sync();
   PHASE_MARK(1);
 
   // (B) Y contraction for every (X node, pixel row ii), column by column. Where
@@ -757,9 +772,14 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
     // the two halves' item counts differ with their windows: both run the
     // larger count, so the synchronisation below is reached by the whole warp
     const int items_u = (LW == 32) ? items : max(items, __shfl_xor_sync(kFull, items, 16));
-    Stride2D ix(lane, s, LW);
-    for (int t0 = 0; t0 < items_u; t0 += LW, ix.next()) {
-      const bool act = t0 + lane < items;
+    // a team's thread keeps its walk over the rows of s (the window's change)
+    auto item_walk = [&] {
+      if constexpr (TW > 0) return *walk;
+      else return Stride2D(lane, s, LW);
+    };
+    Stride2D ix = item_walk();
+    for (int t0 = 0; t0 < items_u; t0 += TS, ix.next()) {
+      const bool act = t0 + t_first < items;
       const int xr = ix.r, py = ix.c;
       float gv[NG];
       if (act) {
@@ -792,7 +812,8 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
           gv[9] = z3[0] * by0 + z3[1] * by1 + z3[2] * by2 + z3[3] * by3;
         }
       }
-      if constexpr (TR::ALIAS) __syncwarp();  // G aliases A (see WarpLayout)
+      // G aliases A (see WarpLayout; a team's maps do not alias)
+      if constexpr (TR::ALIAS && TW == 0) __syncwarp();
       if (act) {
         float* go = G + (xr * s + py) * GP;
         if constexpr (MODE == 6) {
@@ -808,7 +829,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       }
     }
   }
-  __syncwarp();
+  stage_sync();
   PHASE_MARK(2);
 
   // (C) X contraction per pixel, fused with the likelihood sums.
@@ -881,19 +902,20 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
         float dX3 = (h1 - h0) * dx0 + (h2 - h1) * dx1 + (h3 - h2) * dx2;
         float dY3 = q[0][4].x * bx0 + q[1][4].x * bx1 + q[2][4].x * bx2 + q[3][4].x * bx3;
         float dZ3 = q[0][4].y * bx0 + q[1][4].y * bx1 + q[2][4].y * bx2 + q[3][4].y * bx3;
-        // mixture (CPUmleFit_LM.cpp:3311-3322)
+        // mixture (CPUmleFit_LM.cpp:3311-3322), each sum's rounding order written
+        // out: every kernel that includes this gives the same bits
         const float g2 = th[7], h2m = 1.0f - g2;
         const float m5 = bg + N * f, m3 = bg + N * f3;
-        dudt[0] = dudt[0] * g2 + h2m * (-N * dX3);
-        dudt[1] = dudt[1] * g2 + h2m * (-N * dY3);
-        dudt[2] = f * g2 + h2m * f3;
+        dudt[0] = fmaf(dudt[0], g2, h2m * (-N * dX3));
+        dudt[1] = fmaf(h2m, -N * dY3, dudt[1] * g2);
+        dudt[2] = fmaf(f, g2, h2m * f3);
         dudt[3] = g2 + h2m;
-        dudt[4] = (N * dZ) * g2 + h2m * (N * dZ3);
+        dudt[4] = fmaf(N * dZ, g2, h2m * (N * dZ3));
         dudt[5] = N * dW;
         dudt[6] = N * dU;
         // m5 - m3 = N (f5 - f3): formed without the background, which cancels
         dudt[NV - 1] = N * (f - f3);
-        model = m3 * h2m + m5 * g2;
+        model = fmaf(m5, g2, m3 * h2m);
       }
       float d = data[p];
       if constexpr (VAR) {
@@ -915,9 +937,17 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
         } else {
           term = 2.0f * model;
         }
-        er.add(term);
         const float t1 = 1.0f - dm;
         const float t2 = dm * inv;
+        if constexpr (TW > 0) {
+          rec[p] = term;
+          rec[L.s2p + p] = t1;
+          rec[2 * L.s2p + p] = t2;
+#pragma unroll
+          for (int l = 0; l < NV; ++l) rec[(3 + l) * L.s2p + p] = dudt[l];
+          return;
+        }
+        er.add(term);
 #pragma unroll
         for (int l = 0; l < NV; ++l) ac[l] = fmaf(t1, dudt[l], ac[l]);
         int k = NV;
@@ -930,6 +960,16 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       } else {
         // Fisher information and log-likelihood (CPUmleFit_LM.cpp:2730-2742).
         const float im = inv;
+        if constexpr (TW > 0) {
+          float ll = 0.0f;
+          if (model > 0.0f) ll = (d > 0.0f) ? (d * logf(model) - model - d * logf(d) + d) : -model;
+          rec[p] = ll;
+          rec[L.s2p + p] = 0.0f;
+          rec[2 * L.s2p + p] = im;
+#pragma unroll
+          for (int l = 0; l < NV; ++l) rec[(3 + l) * L.s2p + p] = dudt[l];
+          return;
+        }
         int k = NV;
 #pragma unroll
         for (int l = 0; l < NV; ++l) {
@@ -944,8 +984,12 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       }
     };
     if constexpr (LW == 32) {
-      Stride2D ix(lane, s);
-      for (int p = lane; p < s2; p += 32, ix.next()) pixel(p, ix.r, ix.c, err, acc);
+      auto pixel_walk = [&] {
+        if constexpr (TW > 0) return *walk;
+        else return Stride2D(lane, s);
+      };
+      Stride2D ix = pixel_walk();
+      for (int p = t_first; p < s2; p += TS, ix.next()) pixel(p, ix.r, ix.c, err, acc);
     } else {
       Stride2D ia(lane, s), ib(lane + 16, s);
       for (int p = lane; p < s2; p += 32, ia.next(), ib.next()) {
@@ -1136,6 +1180,74 @@ __device__ __forceinline__ float lane_solve(int lane, const float (&lr)[NV], con
   return x;
 }
 
+// CRLB = diag(M^-1) of the Fisher matrix M (the reference inverts it with an
+// unpivoted LU, VC/CPUmleFit_LM/MatInvLib.h:17-77); lane c < NV holds row c in
+// hr and receives the variance of parameter c. Lane-parallel in FP32 on the
+// Jacobi-scaled matrix S = D^-1 M D^-1 (unit diagonal, so its condition number
+// is that of the parameters' correlations, not of their units): Cholesky
+// S = L L^T, then diag(S^-1)_c = sum_k ((L^-1)_kc)^2 with the columns of L^-1 by
+// forward substitution, and (M^-1)_cc = (S^-1)_cc / M_cc. A parameter with an
+// exactly zero Fisher row (zero derivative everywhere) is decoupled: its
+// variance is +inf, the others are unaffected.
+template <int NV>
+__device__ __forceinline__ float fisher_crlb(int lane, const float (&hr)[NV]) {
+  float crlb = 0.0f;  // lane c: variance of parameter c
+  float mr[NV], dk[NV];
+  float mydiag = 0.0f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (lane == k) mydiag = hr[k];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) dk[k] = bcast(mydiag, k);
+  const float sd = sqrtf(mydiag);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const float den = sd * sqrtf(dk[k]);
+    mr[k] = (lane == k) ? 1.0f : ((den > 0.0f) ? hr[k] / den : 0.0f);
+  }
+  float lr[NV], invd = 1.0f;
+  bool okc = true;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) lr[j] = 0.0f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const float ajj = bcast(mr[j], j);
+    if (!(ajj > 0.0f)) okc = false;
+    const float inv = rsqrtf(ajj);
+    const float ljj = ajj * inv;
+    const float lij = (lane > j) ? mr[j] * inv : ((lane == j) ? ljj : 0.0f);
+    lr[j] = lij;
+    if (lane == j) invd = inv;
+#pragma unroll
+    for (int k = j + 1; k < NV; ++k) {
+      const float lkj = bcast(lij, k);
+      if (lane > j && k <= lane) mr[k] = fmaf(-lij, lkj, mr[k]);
+    }
+  }
+  // columns of L^-1: z = L^-1 e_c, lane i holds z_i; accumulate z_i^2 per c
+  float acc[NV];
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    float part = 0.0f, z = 0.0f;
+#pragma unroll
+    for (int k = c; k < NV; ++k) {
+      const float zk = bcast(((k == c ? 1.0f : 0.0f) - part) * invd, k);
+      if (lane == k) z = zk;
+      else if (lane > k) part = fmaf(lr[k], zk, part);
+    }
+    acc[c] = (lane >= c && lane < NV) ? z * z : 0.0f;
+  }
+  warp_sum_array<NV>(acc);
+#pragma unroll
+  for (int c = 0; c < NV; ++c)
+    if (lane == c) crlb = okc ? acc[c] / dk[c] : __int_as_float(0x7fc00000);
+  // decoupled zero rows
+#pragma unroll
+  for (int c = 0; c < NV; ++c)
+    if (lane == c && dk[c] == 0.0f) crlb = __int_as_float(0x7f800000);
+  return crlb;
+}
+
 // Stage one ROI in the warp's shared memory: its pixels (4Pi: the four
 // channel planes, rois laid out [channel][roi][s][s]) and the 4Pi channel
 // offsets dT [roi][channel][6].
@@ -1209,6 +1321,190 @@ __device__ __forceinline__ void initial_guess(const float* data, int s, int lane
   g[3] = (mn > 0.01f) ? mn : 0.01f;
 }
 
+// Initial x, y, N, bg of the ROI staged in ws on lanes 0 .. 3 (other lanes 0).
+template <int MODE>
+__device__ __forceinline__ float start_guess(const WarpLayout& L, const float* ws, int lane) {
+  using TR = ModeTraits<MODE>;
+  float v = 0.0f;
+  if constexpr (TR::NCH == 1) {
+    float g[4];
+    initial_guess(ws, L.s, lane, g);
+    if (lane < 4) v = g[lane];
+  } else {
+    // 4Pi: the mean over the channels of the single-channel rule, the
+    // centroid taken back by the channel's offset.
+    const float* dts = ws + L.off_dt();
+    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int ch = 0; ch < TR::NCH; ++ch) {
+      float g[4];
+      initial_guess(ws + ch * L.s2p, L.s, lane, g);
+      sum[0] += g[0] - dts[ch * TR::NV + 0];
+      sum[1] += g[1] - dts[ch * TR::NV + 1];
+      sum[2] += g[2];
+      sum[3] += g[3];
+    }
+    if (lane < 4) v = sum[lane] / (float)TR::NCH;
+  }
+  return v;
+}
+
+// The fit's first parameters, lane l < NV parameter l: v on lanes 0 .. 3
+// (start_guess), then the start's z, colour, orientation or phase.
+template <int MODE>
+__device__ __forceinline__ float start_params(const FitArgs& a, int lane, int64_t roi, int start,
+                                              float v) {
+  if (MODE == 6) {
+    if (lane == 4) v = (float)a.m.n[2] / 2.0f;
+  } else if (MODE == 7) {
+    const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
+    const bool use = (a.n_starts > 0 || a.m.init_p_len >= 2) && ip[0] != 0.0f;
+    if (lane == 4) v = use ? ip[0] : (float)a.m.n[2] / 2.0f;
+    if (lane == 5) v = use ? ip[1] : (float)a.m.n[3] / 2.0f;
+  } else if (MODE == 8) {
+    // (z, w, u, g2) from initP, shared by all ROIs (CPUmleFit_LM.cpp:3246-3256)
+    const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
+    if (lane >= 4 && lane < 8) v = ip[lane - 4];
+  } else {
+    // 4Pi: per-ROI initial z and phase, one array per start
+    const int64_t i0 = (int64_t)start * a.nfits + roi;
+    if (lane == 4) v = a.z0[i0];
+    if (lane == 5) v = wrap_phase(a.w0[i0], a.m.n[3]);
+  }
+  return v;
+}
+
+// LM state of one fit: per lane, lane l < NV owning parameter l (value, value
+// before the last step, signs and clamps of the last two, fade, value at the
+// last evaluation), and the damping, deviances and switches, equal on every
+// lane.
+struct LmLane {
+  float par, opar, sg, osg, cl, ocl, fd, par_eval;
+  float lambda, olambda, sum_update;
+  FPair err, oerr;
+  int turn;
+};
+
+// |(newErr - oldErr) / newErr| (CPUmleFit_LM.cpp:2565)
+__device__ __forceinline__ float lm_rel_change(const LmLane& st) {
+  const float dhi = st.err.hi - st.oerr.hi;
+  const float dlo = st.err.lo - st.oerr.lo;
+  return fabsf((dhi + dlo) / (st.err.hi + st.err.lo));
+}
+
+template <int MODE>
+__device__ __forceinline__ bool lm_converged(const LmLane& st) {
+  return lm_rel_change(st) < 1e-6f || (MODE == 8 && st.sum_update < 1e-5f);  // :2565, :3355
+}
+
+// Whether the spatial parameters are those of the last evaluation (bitwise), so
+// that its maps serve the Fisher pass.
+template <int MODE>
+__device__ __forceinline__ bool lm_same_place(const LmLane& st, int lane) {
+  constexpr int NV = ModeTraits<MODE>::NV;
+  const bool spatial = lane < NV && lane != 2 && lane != 3 && !(MODE == 8 && lane == 7);
+  const bool same = (MODE == 8) || !spatial || __float_as_uint(st.par) == __float_as_uint(st.par_eval);
+  return __all_sync(kFull, same);
+}
+
+// Takes the last step back when it raised the deviance too far, and sets the
+// damping.
+__device__ __forceinline__ void lm_weigh(LmLane& st) {
+  const float e_new = st.err.hi + st.err.lo, e_old = st.oerr.hi + st.oerr.lo;
+  // newErr > 1.5 * oldErr, evaluated in double by the reference: the FMA
+  // forms 1.5 * oldErr - newErr with one rounding, which keeps its sign.
+  if (fmaf(1.5f, e_old, -e_new) < 0.0f) {
+    st.sg = st.osg;
+    st.cl = st.ocl;
+    st.par = st.opar;
+    st.lambda = st.olambda;
+    st.err = st.oerr;
+    st.lambda = 10.0f * st.lambda;
+  } else if (e_new < e_old) {
+    if (st.lambda > 1.0f)
+      st.lambda = (float)((double)st.lambda * 0.8);
+    else if (st.lambda < 1.0f)
+      st.lambda = 1.0f;
+  }
+}
+
+// Bounds of parameter l on lane l (CPUmleFit_LM.cpp:2626-2634, :3003-3010,
+// :3421-3447).
+template <int MODE>
+__device__ __forceinline__ float lm_bounds(float par, const ModelDev& m, int s, int lane) {
+  if (MODE == 8 && lane < 2) {
+    const float lo = (float)(s - 1) / 2.0f - (float)s / 4.0f;  // exact for s <= 51
+    const float hi = (float)(s - 1) / 2.0f + (float)s / 4.0f;
+    par = (par > lo) ? par : lo;
+    par = (par < hi) ? par : hi;
+  }
+  if (lane == 2) par = (par > 1.0f) ? par : 1.0f;
+  // max(bg, 0.01) in double: no float lies strictly between 0.01f and
+  // 0.01, so the float comparison selects the same branch.
+  if (lane == 3) par = (par > 0.01f) ? par : 0.01f;
+  if (lane == 4) {
+    par = (par > 0.0f) ? par : 0.0f;
+    const float zmax = (MODE == 6) ? (float)(m.n[2] - 4) : (float)m.n[2] - 0.5f;
+    par = (par < zmax) ? par : zmax;
+  }
+  if (MODE == 7 && lane == 5) {
+    par = (par > 0.0f) ? par : 0.0f;
+    const float wmax = (float)m.n[3] - 0.5f;
+    par = (par < wmax) ? par : wmax;
+  }
+  if (MODE == kFit4Pi && lane == 5) par = wrap_phase(par, m.n[3]);
+  if (MODE == 8) {
+    if (lane == 5) {
+      // periodic azimuth (:3436-3443): period nW - 2
+      const int nw = m.n[3];
+      if (par <= 1.0f)
+        par = (float)(nw - 2) + par;
+      else if (par > (float)(nw - 1))
+        par = (2.0f + par) - (float)nw;
+    }
+    if (lane == 6) {
+      par = (par > 1.0f) ? par : 1.0f;
+      const float umax = (float)m.n[4] - 0.5f;
+      par = (par < umax) ? par : umax;
+    }
+    if (lane == 7) {
+      par = (par < 1.0f) ? par : 1.0f;
+      par = (par > 0.0f) ? par : 0.0f;
+    }
+  }
+  return par;
+}
+
+// Takes the step `upd` (lane l < NV: parameter l; fit type 7 scales its colour
+// entry) of a solve that succeeded: clamps, fades and bounds (lm_bounds, or the
+// caller's form of it).
+template <int MODE, class Bounds>
+__device__ __forceinline__ void lm_apply(LmLane& st, const ModelDev& m, int lane, float& upd,
+                                         Bounds&& bounds) {
+  constexpr int NV = ModeTraits<MODE>::NV;
+  if (MODE == 7 && lane == 5) upd = upd * 10.0f;  // CPUmleFit_LM.cpp:2951
+  st.osg = st.sg;
+  st.ocl = st.cl;
+  st.opar = st.par;
+  st.olambda = st.lambda;
+  st.oerr = st.err;
+  if (MODE == 7) {
+    // "let it go" (:2966-2971)
+    const float dz = bcast(upd, 4);
+    if (fabsf(dz) < 0.005f && st.turn) {
+      if (lane == 5) st.cl = st.ocl = (float)m.n[3] / 10.0f;
+      if (lane == 4) st.cl = st.ocl = 2.0f;
+      st.turn = 0;
+    }
+  }
+  if (st.sg != 0.0f) {
+    if ((st.sg == 1.0f && upd < 0.0f) || (st.sg == -1.0f && upd > 0.0f)) st.cl = st.cl * st.fd;
+  }
+  st.sg = (upd > 0.0f) ? 1.0f : -1.0f;
+  const float step = upd / (1.0f + fabsf(upd / st.cl));
+  if (MODE == 8) st.sum_update = warp_sum(lane < NV ? fabsf(step) : 0.0f);
+  st.par = bounds(st.par - step);
+}
+
 // Result of one fit, distributed like the LM state: lane l < NV holds
 // parameter l and its variance; the log-likelihood and the iteration count are
 // on every lane.
@@ -1229,60 +1525,15 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
   PHASE_DECL();
   // Initial guesses (CPUgaussLib.cpp:172-225, CPUmleFit_LM.cpp:2477-2482),
   // then lane l keeps parameter l.
-  float par;
-  {
-    float v = 0.0f;
-    if constexpr (TR::NCH == 1) {
-      float g[4];
-      initial_guess(ws, s, lane, g);
-      if (lane < 4) v = g[lane];
-    } else {
-      // 4Pi: the mean over the channels of the single-channel rule, the
-      // centroid taken back by the channel's offset.
-      const float* dts = ws + L.off_dt();
-      float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      for (int ch = 0; ch < TR::NCH; ++ch) {
-        float g[4];
-        initial_guess(ws + ch * L.s2p, s, lane, g);
-        sum[0] += g[0] - dts[ch * NV + 0];
-        sum[1] += g[1] - dts[ch * NV + 1];
-        sum[2] += g[2];
-        sum[3] += g[3];
-      }
-      if (lane < 4) v = sum[lane] / (float)TR::NCH;
-    }
-    if (MODE == 6) {
-      if (lane == 4) v = (float)a.m.n[2] / 2.0f;
-    } else if (MODE == 7) {
-      const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
-      const bool use = (a.n_starts > 0 || a.m.init_p_len >= 2) && ip[0] != 0.0f;
-      if (lane == 4) v = use ? ip[0] : (float)a.m.n[2] / 2.0f;
-      if (lane == 5) v = use ? ip[1] : (float)a.m.n[3] / 2.0f;
-    } else if (MODE == 8) {
-      // (z, w, u, g2) from initP, shared by all ROIs (CPUmleFit_LM.cpp:3246-3256)
-      const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
-      if (lane >= 4 && lane < 8) v = ip[lane - 4];
-    } else {
-      // 4Pi: per-ROI initial z and phase, one array per start
-      const int64_t i0 = (int64_t)start * a.nfits + roi;
-      if (lane == 4) v = a.z0[i0];
-      if (lane == 5) v = wrap_phase(a.w0[i0], a.m.n[3]);
-    }
-    par = v;
-  }
+  const float par0 = start_params<MODE>(a, lane, roi, start, start_guess<MODE>(L, ws, lane));
 
   // Per-lane LM state (CPUmleFit_LM.cpp:2425-2450): lane l < NV owns
   // parameter l.
-  float opar = par, sg = 0.0f, osg = 0.0f, cl, fd, par_eval = par;
-  clamp_fade<MODE>(lane, cl, fd);
-  float ocl = cl;
+  float cl0, fd0;
+  clamp_fade<MODE>(lane, cl0, fd0);
+  LmLane st{par0, par0, 0.0f, 0.0f, cl0, cl0, fd0, par0, 1.0f, 1.0f, 1e10f, {1e12f, 0.0f}, {1e13f, 0.0f}, 1};
   float gl = 0.0f;   // gradient entry
   float hr[NV];      // Hessian row (damped in place), or the Fisher row
-  // Warp-uniform state.
-  float lambda = 1.0f, olambda = 1.0f, sum_update = 1e10f;
-  FPair err{1e12f, 0.0f}, oerr{1e13f, 0.0f};
-  int turn = 1;
-
   // One evaluation call site for the initial pass, every accepted step and the
   // final CRLB pass (keeps the kernel's instruction footprint small).
   int kk = 0;
@@ -1303,16 +1554,12 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
       // alone. After a rejected step the position differs and the pass is
       // complete. Bitwise equality, so the results are those of a full pass.
       bool maps_ready = false;
-      if (fisher && TR::NCH == 1) {
-        const bool spatial = lane < NV && lane != 2 && lane != 3 && !(MODE == 8 && lane == 7);
-        const bool same = (MODE == 8) || !spatial || __float_as_uint(par) == __float_as_uint(par_eval);
-        maps_ready = __all_sync(kFull, same);
-      }
-      if (!fisher) par_eval = par;
+      if (fisher && TR::NCH == 1) maps_ready = lm_same_place<MODE>(st, lane);
+      if (!fisher) st.par_eval = st.par;
       float the[NV];
 #pragma unroll
       for (int k = 0; k < NV; ++k)
-        the[k] = bcast((MODE == 8 && fisher && k != 2 && k != 3) ? par_eval : par, k);
+        the[k] = bcast((MODE == 8 && fisher && k != 2 && k != 3) ? st.par_eval : st.par, k);
       evaluate<MODE, VAR, STG>(a, L, ws, lane, the, first && MODE == 7, fisher, e, gl, hr,
                                maps_ready);
       first = false;
@@ -1321,7 +1568,7 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
         ll = e;
         break;
       }
-      err = e;
+      st.err = e;
       PHASE_RESET();
     }
     if (kk >= a.iterations) {
@@ -1332,46 +1579,26 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
     float* rec = (a.trace && start == 0 && kk < a.trace_max && lane == 0)
                      ? a.trace + (roi * (int64_t)a.trace_max + kk) * TRACE_REC
                      : nullptr;
-    // |(newErr - oldErr) / newErr| < 1e-6 (CPUmleFit_LM.cpp:2565)
-    {
-      const float dhi = err.hi - oerr.hi;
-      const float dlo = err.lo - oerr.lo;
-      const float rel = fabsf((dhi + dlo) / (err.hi + err.lo));
-      if (rec) {
-        rec[0] = (float)kk;
-        rec[1] = rel;
-        rec[2] = err.hi + err.lo;
-        rec[3] = oerr.hi + oerr.lo;
-        rec[4] = 0.0f;
-      }
-      if (rel < 1e-6f || (MODE == 8 && sum_update < 1e-5f)) {  // :3355
-        if (rec) rec[4] = 1.0f;
-        fisher = true;
-        need_eval = true;
-        continue;
-      }
+    const bool stop = lm_converged<MODE>(st);
+    if (rec) {
+      rec[0] = (float)kk;
+      rec[1] = lm_rel_change(st);
+      rec[2] = st.err.hi + st.err.lo;
+      rec[3] = st.oerr.hi + st.oerr.lo;
+      rec[4] = stop ? 1.0f : 0.0f;
     }
-    const float e_new = err.hi + err.lo, e_old = oerr.hi + oerr.lo;
-    // newErr > 1.5 * oldErr, evaluated in double by the reference: the FMA
-    // forms 1.5 * oldErr - newErr with one rounding, which keeps its sign.
-    if (fmaf(1.5f, e_old, -e_new) < 0.0f) {
-      sg = osg;
-      cl = ocl;
-      par = opar;
-      lambda = olambda;
-      err = oerr;
-      lambda = 10.0f * lambda;
-    } else if (e_new < e_old) {
-      if (lambda > 1.0f)
-        lambda = (float)((double)lambda * 0.8);
-      else if (lambda < 1.0f)
-        lambda = 1.0f;
+    if (stop) {
+      fisher = true;
+      need_eval = true;
+      continue;
     }
+    const float e_new = st.err.hi + st.err.lo, e_old = st.oerr.hi + st.oerr.lo;  // for the record
+    lm_weigh(st);
     // H_ll *= lambda, in place (cumulative across failed solves, as in the
     // reference).
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-      if (lane == k) hr[k] *= lambda;
+      if (lane == k) hr[k] *= st.lambda;
     // A parameter whose derivative is exactly zero at every pixel (z on the
     // mirror-padded boundary knot) has an exactly zero Hessian row. The
     // reference only survives that case through rounding noise of its double
@@ -1445,79 +1672,17 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
       }
     }
     if (ok) {
-      if (MODE == 7 && lane == 5) upd = upd * 10.0f;  // :2951
-      osg = sg;
-      ocl = cl;
-      opar = par;
-      olambda = lambda;
-      oerr = err;
-      if (MODE == 7) {
-        // "let it go" (:2966-2971)
-        const float dz = bcast(upd, 4);
-        if (fabsf(dz) < 0.005f && turn) {
-          if (lane == 5) cl = ocl = (float)a.m.n[3] / 10.0f;
-          if (lane == 4) cl = ocl = 2.0f;
-          turn = 0;
-        }
-      }
-      if (sg != 0.0f) {
-        if ((sg == 1.0f && upd < 0.0f) || (sg == -1.0f && upd > 0.0f)) cl = cl * fd;
-      }
-      sg = (upd > 0.0f) ? 1.0f : -1.0f;
-      const float step = upd / (1.0f + fabsf(upd / cl));
-      par = par - step;
-      if (MODE == 8) sum_update = warp_sum(lane < NV ? fabsf(step) : 0.0f);
-      // Bounds (CPUmleFit_LM.cpp:2626-2634, :3003-3010, :3421-3447).
-      if (MODE == 8 && lane < 2) {
-        const float lo = (float)(s - 1) / 2.0f - (float)s / 4.0f;  // exact for s <= 51
-        const float hi = (float)(s - 1) / 2.0f + (float)s / 4.0f;
-        par = (par > lo) ? par : lo;
-        par = (par < hi) ? par : hi;
-      }
-      if (lane == 2) par = (par > 1.0f) ? par : 1.0f;
-      // max(bg, 0.01) in double: no float lies strictly between 0.01f and
-      // 0.01, so the float comparison selects the same branch.
-      if (lane == 3) par = (par > 0.01f) ? par : 0.01f;
-      if (lane == 4) {
-        par = (par > 0.0f) ? par : 0.0f;
-        const float zmax = (MODE == 6) ? (float)(a.m.n[2] - 4) : (float)a.m.n[2] - 0.5f;
-        par = (par < zmax) ? par : zmax;
-      }
-      if (MODE == 7 && lane == 5) {
-        par = (par > 0.0f) ? par : 0.0f;
-        const float wmax = (float)a.m.n[3] - 0.5f;
-        par = (par < wmax) ? par : wmax;
-      }
-      if (MODE == kFit4Pi && lane == 5) par = wrap_phase(par, a.m.n[3]);
-      if (MODE == 8) {
-        if (lane == 5) {
-          // periodic azimuth (:3436-3443): period nW - 2
-          const int nw = a.m.n[3];
-          if (par <= 1.0f)
-            par = (float)(nw - 2) + par;
-          else if (par > (float)(nw - 1))
-            par = (2.0f + par) - (float)nw;
-        }
-        if (lane == 6) {
-          par = (par > 1.0f) ? par : 1.0f;
-          const float umax = (float)a.m.n[4] - 0.5f;
-          par = (par < umax) ? par : umax;
-        }
-        if (lane == 7) {
-          par = (par < 1.0f) ? par : 1.0f;
-          par = (par > 0.0f) ? par : 0.0f;
-        }
-      }
+      lm_apply<MODE>(st, a.m, lane, upd, [&](float p) { return lm_bounds<MODE>(p, a.m, s, lane); });
       need_eval = true;
     } else {
-      lambda = 10.0f * lambda;
+      st.lambda = 10.0f * st.lambda;
     }
     if (a.trace) {
       // decision record (diagnostics): gathered from the parameter lanes
 #pragma unroll
       for (int k = 0; k < NV; ++k) {
         const float uk = bcast(ok ? upd : 0.0f, k);
-        const float pk = bcast(par, k);
+        const float pk = bcast(st.par, k);
         if (rec) {
           rec[6 + k] = uk;
           rec[14 + k] = pk;
@@ -1525,7 +1690,7 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
       }
       if (rec) {
         rec[4] = (e_new > 1.5f * e_old ? 2.0f : 0.0f) + (e_new < e_old ? 4.0f : 0.0f) + (ok ? 8.0f : 0.0f);
-        rec[5] = lambda;
+        rec[5] = st.lambda;
         rec[22] = 0.0f;
       }
     }
@@ -1533,73 +1698,10 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
     PHASE_MARK(6);
   }
 
-  // CRLB = diag(M^-1) of the Fisher matrix M (the reference inverts it with an
-  // unpivoted LU, VC/CPUmleFit_LM/MatInvLib.h:17-77). Here, lane-parallel in
-  // FP32 on the Jacobi-scaled matrix S = D^-1 M D^-1 (unit diagonal, so its
-  // condition number is that of the parameters' correlations, not of their
-  // units): Cholesky S = L L^T, then diag(S^-1)_c = sum_k ((L^-1)_kc)^2 with the
-  // columns of L^-1 by forward substitution, and (M^-1)_cc = (S^-1)_cc / M_cc.
-  // A parameter with an exactly zero Fisher row (zero derivative everywhere)
-  // is decoupled: its variance is +inf, the others are unaffected.
   PHASE_RESET();
-  float crlb = 0.0f;  // lane c: variance of parameter c
-  {
-    float mr[NV], dk[NV];
-    float mydiag = 0.0f;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-      if (lane == k) mydiag = hr[k];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) dk[k] = bcast(mydiag, k);
-    const float sd = sqrtf(mydiag);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const float den = sd * sqrtf(dk[k]);
-      mr[k] = (lane == k) ? 1.0f : ((den > 0.0f) ? hr[k] / den : 0.0f);
-    }
-    float lr[NV], invd = 1.0f;
-    bool okc = true;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) lr[j] = 0.0f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const float ajj = bcast(mr[j], j);
-      if (!(ajj > 0.0f)) okc = false;
-      const float inv = rsqrtf(ajj);
-      const float ljj = ajj * inv;
-      const float lij = (lane > j) ? mr[j] * inv : ((lane == j) ? ljj : 0.0f);
-      lr[j] = lij;
-      if (lane == j) invd = inv;
-#pragma unroll
-      for (int k = j + 1; k < NV; ++k) {
-        const float lkj = bcast(lij, k);
-        if (lane > j && k <= lane) mr[k] = fmaf(-lij, lkj, mr[k]);
-      }
-    }
-    // columns of L^-1: z = L^-1 e_c, lane i holds z_i; accumulate z_i^2 per c
-    float acc[NV];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      float part = 0.0f, z = 0.0f;
-#pragma unroll
-      for (int k = c; k < NV; ++k) {
-        const float zk = bcast(((k == c ? 1.0f : 0.0f) - part) * invd, k);
-        if (lane == k) z = zk;
-        else if (lane > k) part = fmaf(lr[k], zk, part);
-      }
-      acc[c] = (lane >= c && lane < NV) ? z * z : 0.0f;
-    }
-    warp_sum_array<NV>(acc);
-#pragma unroll
-    for (int c = 0; c < NV; ++c)
-      if (lane == c) crlb = okc ? acc[c] / dk[c] : __int_as_float(0x7fc00000);
-    // decoupled zero rows
-#pragma unroll
-    for (int c = 0; c < NV; ++c)
-      if (lane == c && dk[c] == 0.0f) crlb = __int_as_float(0x7f800000);
-  }
+  const float crlb = fisher_crlb<NV>(lane, hr);
   PHASE_MARK(7);
-  return RoiResult{par, crlb, ll.hi + ll.lo, kk};
+  return RoiResult{st.par, crlb, ll.hi + ll.lo, kk};
 }
 
 template <int MODE>

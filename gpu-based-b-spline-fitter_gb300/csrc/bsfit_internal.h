@@ -181,17 +181,22 @@ int fit64_smem_bytes(int mode);
 int warp_smem_floats(int mode, int s, bool var = false, int stg = 0);
 cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t stream);
 cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream);
+// The fit with one block per ROI, where that is the faster form (few ROIs);
+// otherwise *taken stays false and nothing is launched.
+cudaError_t launch_team(const FitArgs& a, bool* taken, cudaStream_t stream);
 // Double-float parity-grade fit of fit types 6, 7, 8 (plain ROIs, one start).
 cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream);
 int fitdd_smem_floats(int mode, int s);
 // One double-float evaluation per ROI (double outputs, layout of launch_eval).
 cudaError_t launch_evaldd(const FitArgs& a, const float* theta, double* out, int fisher,
                           cudaStream_t stream);
+// Multiprocessors of a device (asked once per process).
+cudaError_t sm_count(int dev, int* sms);
 // Launch shape of a fitter kernel (warps per block among 4, 2, 1 keeping the
 // most warps resident; blocks per SM; SM count), cached per kernel, size and
 // device.
 cudaError_t pick_launch(const void* kern, int per_warp, int* wpb, int* bps, int* sms);
-// The same with the warps per block forced (force_wpb 1, 2 or 4; 0 chooses).
+// The same with the warps per block forced (force_wpb a power of two; 0 chooses).
 cudaError_t pick_launch_wpb(const void* kern, int per_warp, int force_wpb, int* wpb, int* bps,
                             int* sms);
 
