@@ -170,35 +170,38 @@ cudaError_t pick_launch_wpb(const void* kern, int per_warp, int force_wpb, int* 
   return cudaSuccess;
 }
 
+unsigned long long* WorkCounter::get(cudaStream_t stream) {
+  stream_ = stream;
+  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p_), sizeof(*p_), stream);
+  if (e != cudaSuccess) p_ = nullptr;
+  if (e == cudaSuccess) {
+    e = cudaMemsetAsync(p_, 0, sizeof(*p_), stream);
+    if (e != cudaSuccess) {
+      cudaFreeAsync(p_, stream);
+      p_ = nullptr;
+    }
+  }
+  // Only a failed pool allocation's or memset's own error is cleared (an error
+  // the caller's earlier asynchronous work left pending is not touched
+  // otherwise).
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return p_;
+}
+
+WorkCounter::~WorkCounter() {
+  if (p_) cudaFreeAsync(p_, stream_);
+}
+
 cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t stream) {
   if (a.nseg <= 0) return cudaSuccess;
-  void (*kern)(const BatchArgs) = nullptr;
   const bool cap = a.warp_rois > 0;
-  constexpr int M6 = BSFIT_MINBLOCKS(6), M7 = BSFIT_MINBLOCKS(7), M8 = BSFIT_MINBLOCKS(8);
-  if (cap) {
-    // the capped form of the default kernel (the serving loop's priority launches)
-    if (mode == 6 && !multi) kern = batch_kernel<6, false, M6, 0, true>;
-    else if (mode == 7) kern = multi ? batch_kernel<7, true, M7, 0, true> : batch_kernel<7, false, M7, 0, true>;
-    else if (mode == 8) kern = multi ? batch_kernel<8, true, M8, 0, true> : batch_kernel<8, false, M8, 0, true>;
-    else return cudaErrorInvalidValue;
-  } else if (mode == 6 && !multi) {
-    kern = batch_kernel<6>;
-  } else if (mode == 7) {
-    kern = multi ? batch_kernel<7, true> : batch_kernel<7>;
-  } else if (mode == 8) {
-    kern = multi ? batch_kernel<8, true> : batch_kernel<8>;
-  } else {
-    return cudaErrorInvalidValue;
-  }
   // the autotuner's configuration for the largest ROI size of the batch (the
   // capped form keeps the default kernel and takes the tuner's warps per block)
   TuneConfig tc{0, 0};
   int dev = 0;
-  if (!multi && cudaGetDevice(&dev) == cudaSuccess && tune_lookup(mode, a.s_max, dev, &tc) &&
-      tc.variant > 0) {
-    if (cap) tc.variant = 0;
-    else kern = batch_variant(mode, tc.variant);
-  }
+  if (!multi && cudaGetDevice(&dev) == cudaSuccess) tune_lookup(mode, a.s_max, dev, &tc);
+  if (cap) tc.variant = 0;
+  BatchKern kern = tc.variant > 0 ? batch_variant(mode, tc.variant) : batch_kern_default(mode, multi, cap);
   if (!kern) return cudaErrorInvalidValue;
   const int rpw = tune_rois_per_warp(mode, tc.variant);
   const int per_warp = tune_warp_floats(mode, tc.variant, a.s_max, false) * 4;
@@ -210,6 +213,11 @@ cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t 
   int64_t total = 0;
   for (int i = 0; i < a.nseg; ++i) total += a.seg[i].n;
   int64_t grid = (int64_t)sms * blocks_per_sm;
+  if (tc.variant <= 0 && !cap) {
+    bool taken = false;
+    e = launch_slots_batch(a, mode, multi, multi ? 0 : tc.wpb, total, grid * wpb, &taken, stream);
+    if (taken || e != cudaSuccess) return e;
+  }
   const int64_t need = (total + rpw * wpb - 1) / (rpw * wpb);
   if (need < grid) grid = need;
   // capped: enough blocks that every ROI is fitted
@@ -424,35 +432,20 @@ cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream) {
   const int smem = per_warp * wpb;
   int64_t need = (a.nfits + rpw * wpb - 1) / (rpw * wpb);
   int64_t grid = (int64_t)sms * blocks_per_sm;
+  if (tc.variant <= 0 && !a.trace && !a.flags) {
+    bool taken = false;
+    e = launch_slots(a, tunable ? tc.wpb : 0, grid * wpb, &taken, stream);
+    if (taken || e != cudaSuccess) return e;
+  }
   if (need < grid) grid = need;
   // More ROIs than resident warps: claim them dynamically (iteration counts
   // vary per ROI, and a fixed share per warp leaves the launch waiting on its
-  // slowest warp). The counter comes from the stream-ordered pool; without it
-  // the fixed schedule runs.
+  // slowest warp). Without a counter the fixed schedule runs.
   FitArgs b = a;
-  unsigned long long* claim = nullptr;
-  if (need > grid) {
-    cudaError_t ea = cudaMallocAsync(reinterpret_cast<void**>(&claim), sizeof(*claim), stream);
-    if (ea == cudaSuccess) {
-      ea = cudaMemsetAsync(claim, 0, sizeof(*claim), stream);
-      if (ea == cudaSuccess) {
-        b.claim = claim;
-      } else {
-        cudaFreeAsync(claim, stream);
-        claim = nullptr;
-      }
-    } else {
-      claim = nullptr;
-    }
-    // A failed pool allocation or memset leaves the fixed schedule; only then
-    // is the error it recorded cleared (an error the caller's earlier
-    // asynchronous work left pending is not touched otherwise).
-    if (ea != cudaSuccess) (void)cudaGetLastError();
-  }
+  WorkCounter claim;
+  if (need > grid) b.claim = claim.get(stream);
   kern<<<(unsigned)grid, 32 * wpb, smem, stream>>>(b);
-  e = cudaGetLastError();
-  if (claim) cudaFreeAsync(claim, stream);
-  return e;
+  return cudaGetLastError();
 }
 
 }  // namespace bsfit

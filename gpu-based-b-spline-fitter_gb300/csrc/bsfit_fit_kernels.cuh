@@ -86,6 +86,21 @@ __device__ __forceinline__ void cp_async4(float* dst_smem, const float* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
+// The warp's copy of n floats, the lanes on consecutive ones.
+__device__ __forceinline__ void cp_async_warp(float* dst_smem, const float* src, int n, int lane) {
+  dst_smem += lane;
+  src += lane;
+  int i = n - lane;  // floats left for this lane's positions 0, 32, 64, ...
+  for (; i > 96; i -= 128, dst_smem += 128, src += 128) {
+    cp_async4(dst_smem, src);
+    cp_async4(dst_smem + 32, src + 32);
+    cp_async4(dst_smem + 64, src + 64);
+    cp_async4(dst_smem + 96, src + 96);
+  }
+  if (i > 0) cp_async4(dst_smem, src);
+  if (i > 32) cp_async4(dst_smem + 32, src + 32);
+  if (i > 64) cp_async4(dst_smem + 64, src + 64);
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
@@ -115,7 +130,7 @@ struct ModeTraits<7> {
   static constexpr int NA = 3;  // value, d/dz, d/dw
   static constexpr int NG = 4;  // value, d/dY, d/dz, d/dw
   static constexpr int NCH = 1;
-  static constexpr bool ALIAS = false;
+  static constexpr bool ALIAS = true;
   static constexpr bool TRIM_RS = true;
 };
 // 4Pi: the 4D evaluation of fit type 7 once per channel.
@@ -153,7 +168,7 @@ struct ModeTraits<8> {
 // The stage-A maps (NA per lateral node) and the stage-B maps (NG per X node
 // and pixel row) are both stored by X node ("column"): A column xr holds
 // NA x WP floats, G column xr holds NG x s. For the models whose maps would
-// otherwise bound the warps per SM by shared memory (3D, 5D), the two share
+// otherwise bound the warps per SM by shared memory (3D, 4D, 5D), the two share
 // one region: stage B reads only A column xr to write G column xr and walks the
 // columns in order, so G is written over A columns already consumed. With G
 // at the start of the region and A at offset a_rel with
@@ -220,7 +235,7 @@ __host__ __device__ constexpr WarpLayout make_layout(int mode, int s, bool var =
   L.ng = mode == 6 ? 3 : (mode == 7 || mode == kFit4Pi) ? 4 : 10;
   L.nch = mode == kFit4Pi ? k4PiChannels : 1;
   L.nvar = var ? L.nch : 0;
-  L.alias = mode == 6 || mode == 8;
+  L.alias = mode != kFit4Pi;
   L.stage = (stg && mode == 8) ? kStageFloats : 0;
   return L;
 }
@@ -293,11 +308,25 @@ __device__ __forceinline__ int small_div(int a, int b) {
 // threads): avoids a runtime integer division per item.
 struct Stride2D {
   int r, c, dr, dc, w;
+  Stride2D() = default;
   __device__ __forceinline__ Stride2D(int lane, int w_, int step = 32) : w(w_) {
     r = small_div(lane, w);
     c = lane - r * w;
     dr = small_div(step, w);
     dc = step - dr * w;
+  }
+  // packed into one register (all four below 64) and back
+  __device__ __forceinline__ unsigned pack() const {
+    return (unsigned)r | (unsigned)c << 8 | (unsigned)dr << 16 | (unsigned)dc << 24;
+  }
+  static __device__ __forceinline__ Stride2D unpack(unsigned p, int w) {
+    Stride2D x;
+    x.r = (int)(p & 255u);
+    x.c = (int)((p >> 8) & 255u);
+    x.dr = (int)((p >> 16) & 255u);
+    x.dc = (int)(p >> 24);
+    x.w = w;
+    return x;
   }
   __device__ __forceinline__ void next() {
     r += dr;
@@ -339,14 +368,17 @@ __device__ __forceinline__ float wrap_phase(float w, int nw) {
 // writes each pixel's terms to rec (field f of pixel p at rec[f * L.s2p + p]:
 // the deviance or log-likelihood term, t1, t2, then the NV derivatives) instead
 // of summing them; the team then forms the same sums from the records.
-template <int MODE, int KP, bool VAR, int STG = 0, int LW = 32, int TW = 0>
-__device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout& L, float* ws,
+//
+// ASYNC: the pixels may still be on their way to shared memory (cp.async).
+template <int MODE, int KP, bool VAR, int STG = 0, int LW = 32, int TW = 0, bool ASYNC = false, class Args>
+__device__ __forceinline__ void channel_pass(const Args& a, const WarpLayout& L, float* ws,
                                              const float* data, int lane, const float* th,
                                              bool dup45, bool FISHER, FPair& err,
                                              float (&acc)[KP], FPair& err2, float (&acc2)[KP],
                                              unsigned gm = kFull, bool maps_ready = false,
                                              float* kws = nullptr, float* rec = nullptr,
-                                             int tt = 0, const Stride2D* walk = nullptr) {
+                                             int tt = 0, const Stride2D* walk = nullptr,
+                                             unsigned walk1 = 0) {
   static_assert(LW == 32 || (LW == 16 && MODE == 6 && !VAR && STG == 0),
                 "half-warp ROIs: the 3D EMCCD model only");
   static_assert(TW == 0 || (LW == 32 && STG == 0), "a team is made of whole warps");
@@ -362,6 +394,14 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
   // this thread's first item and the item stride of the shared stages
   const int t_first = (TW > 0) ? tt : lane;
   constexpr int TS = (TW > 0) ? 32 * TW : LW;
+  // The walk over rows of s (stage B's items, the pixels): a team's thread and,
+  // packed, a lane of the slot form keep theirs (the lateral nodes' rows change
+  // with the window).
+  auto row_walk = [&] {
+    if constexpr (TW > 0) return *walk;
+    else if constexpr (ASYNC) return Stride2D::unpack(walk1, s);
+    else return Stride2D(lane, s, LW);
+  };
   auto stage_sync = [] {
     if constexpr (TW > 0) __syncthreads();
     else __syncwarp();
@@ -772,12 +812,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
     // the two halves' item counts differ with their windows: both run the
     // larger count, so the synchronisation below is reached by the whole warp
     const int items_u = (LW == 32) ? items : max(items, __shfl_xor_sync(kFull, items, 16));
-    // a team's thread keeps its walk over the rows of s (the window's change)
-    auto item_walk = [&] {
-      if constexpr (TW > 0) return *walk;
-      else return Stride2D(lane, s, LW);
-    };
-    Stride2D ix = item_walk();
+    Stride2D ix = row_walk();
     for (int t0 = 0; t0 < items_u; t0 += TS, ix.next()) {
       const bool act = t0 + t_first < items;
       const int xr = ix.r, py = ix.c;
@@ -829,6 +864,7 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
       }
     }
   }
+  if constexpr (ASYNC) cp_async_wait_all();  // this lane's pixels have landed
   stage_sync();
   PHASE_MARK(2);
 
@@ -926,10 +962,13 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
         d += v;
       }
       const float inv = __frcp_rn(model);
+      // term: deviance (CPUmleFit_LM.cpp:2540-2559) or log-likelihood
+      // (:2730-2742); t1, t2: the factors of the gradient and of the Hessian, or
+      // nothing and that of the Fisher information. One reciprocal: d / m =
+      // d * (1 / m) and log(m / d) = -log(d / m).
+      float term, t1 = 0.0f, t2 = inv;
+      bool counts = true;
       if (!FISHER) {
-        // CPUmleFit_LM.cpp:2540-2559, with one reciprocal: d / m = d * (1 / m)
-        // and log(m / d) = -log(d / m).
-        float term;
         float dm = 0.0f;
         if (d > 0.0f) {
           dm = d * inv;
@@ -937,17 +976,21 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
         } else {
           term = 2.0f * model;
         }
-        const float t1 = 1.0f - dm;
-        const float t2 = dm * inv;
-        if constexpr (TW > 0) {
-          rec[p] = term;
-          rec[L.s2p + p] = t1;
-          rec[2 * L.s2p + p] = t2;
+        t1 = 1.0f - dm;
+        t2 = dm * inv;
+      } else {
+        counts = model > 0.0f;
+        term = 0.0f;
+        if (counts) term = (d > 0.0f) ? (d * logf(model) - model - d * logf(d) + d) : -model;
+      }
+      if constexpr (TW > 0) {
+        rec[p] = term;
+        rec[L.s2p + p] = t1;
+        rec[2 * L.s2p + p] = t2;
 #pragma unroll
-          for (int l = 0; l < NV; ++l) rec[(3 + l) * L.s2p + p] = dudt[l];
-          return;
-        }
-        er.add(term);
+        for (int l = 0; l < NV; ++l) rec[(3 + l) * L.s2p + p] = dudt[l];
+      } else {
+        if (counts) er.add(term);
 #pragma unroll
         for (int l = 0; l < NV; ++l) ac[l] = fmaf(t1, dudt[l], ac[l]);
         int k = NV;
@@ -957,38 +1000,10 @@ __device__ __forceinline__ void channel_pass(const FitArgs& a, const WarpLayout&
 #pragma unroll
           for (int mm = l; mm < NV; ++mm, ++k) ac[k] = fmaf(tl, dudt[mm], ac[k]);
         }
-      } else {
-        // Fisher information and log-likelihood (CPUmleFit_LM.cpp:2730-2742).
-        const float im = inv;
-        if constexpr (TW > 0) {
-          float ll = 0.0f;
-          if (model > 0.0f) ll = (d > 0.0f) ? (d * logf(model) - model - d * logf(d) + d) : -model;
-          rec[p] = ll;
-          rec[L.s2p + p] = 0.0f;
-          rec[2 * L.s2p + p] = im;
-#pragma unroll
-          for (int l = 0; l < NV; ++l) rec[(3 + l) * L.s2p + p] = dudt[l];
-          return;
-        }
-        int k = NV;
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const float tl = dudt[l] * im;
-#pragma unroll
-          for (int mm = l; mm < NV; ++mm, ++k) ac[k] = fmaf(tl, dudt[mm], ac[k]);
-        }
-        if (model > 0.0f) {
-          float ll = (d > 0.0f) ? (d * logf(model) - model - d * logf(d) + d) : -model;
-          er.add(ll);
-        }
       }
     };
     if constexpr (LW == 32) {
-      auto pixel_walk = [&] {
-        if constexpr (TW > 0) return *walk;
-        else return Stride2D(lane, s);
-      };
-      Stride2D ix = pixel_walk();
+      Stride2D ix = row_walk();
       for (int p = t_first; p < s2; p += TS, ix.next()) pixel(p, ix.r, ix.c, err, acc);
     } else {
       Stride2D ia(lane, s), ib(lane + 16, s);
@@ -1137,7 +1152,10 @@ __device__ __forceinline__ void chol_solve(const float (&u)[NV * NV], const floa
 // refinement), and every per-parameter rule is one lane's instruction stream.
 // The decisions (convergence, accept / reject, damping) are warp-uniform.
 
-__device__ __forceinline__ float bcast(float v, int k) { return __shfl_sync(kFull, v, k); }
+template <int W = 32>
+__device__ __forceinline__ float bcast(float v, int k) {
+  return __shfl_sync(kFull, v, k, W);
+}
 
 // Initial clamp and fade of parameter l (CPUmleFit_LM.cpp:2434, :2786-2788,
 // :3191-3193).
@@ -1159,21 +1177,22 @@ __device__ __forceinline__ void clamp_fade(int l, float& c, float& f) {
 }
 
 // Lane-parallel solve of (L L^T) x = b: lane i holds b_i, row i of L (lr),
-// column i of L below the diagonal (lc[k] = L[k][i]) and 1 / L_ii.
-template <int NV>
+// column i of L below the diagonal (lc[k] = L[k][i]) and 1 / L_ii. W: lanes of
+// one system (32, or 8 for four systems side by side, `lane` counted within one).
+template <int NV, int W = 32>
 __device__ __forceinline__ float lane_solve(int lane, const float (&lr)[NV], const float (&lc)[NV],
                                             float invd, float b) {
   float y = b;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const float yk = bcast(y * invd, k);
+    const float yk = bcast<W>(y * invd, k);
     if (lane == k) y = yk;
     else if (lane > k) y = fmaf(-lr[k], yk, y);
   }
   float x = y;
 #pragma unroll
   for (int k = NV - 1; k >= 0; --k) {
-    const float xk = bcast(x * invd, k);
+    const float xk = bcast<W>(x * invd, k);
     if (lane == k) x = xk;
     else if (lane < k) x = fmaf(-lc[k], xk, x);
   }
@@ -1251,8 +1270,8 @@ __device__ __forceinline__ float fisher_crlb(int lane, const float (&hr)[NV]) {
 // Stage one ROI in the warp's shared memory: its pixels (4Pi: the four
 // channel planes, rois laid out [channel][roi][s][s]) and the 4Pi channel
 // offsets dT [roi][channel][6].
-template <int MODE, bool VAR = false>
-__device__ __forceinline__ void load_roi(const FitArgs& a, const WarpLayout& L, float* ws,
+template <int MODE, bool VAR = false, class Args>
+__device__ __forceinline__ void load_roi(const Args& a, const WarpLayout& L, float* ws,
                                          int lane, int64_t roi) {
   const int s2 = L.s * L.s;
   const int nch = ModeTraits<MODE>::NCH;
@@ -1321,6 +1340,85 @@ __device__ __forceinline__ void initial_guess(const float* data, int s, int lane
   g[3] = (mn > 0.01f) ? mn : 0.01f;
 }
 
+// The LM step's solve, lane-parallel: H upd = g with row l of the damped Hessian
+// (hr) and gradient entry l on lane l < NV; W: lanes of one system (32, or 8 for
+// four systems side by side, `lane` counted within one). ok: whether the
+// factorisation succeeded and, but for fit type 6, gave numbers.
+//
+// A parameter whose derivative is exactly zero at every pixel (z on the
+// mirror-padded boundary knot) has an exactly zero Hessian row. The reference
+// only survives that case through rounding noise of its double derivative sums
+// (a ~1e-29 pivot and a huge step of noise-determined sign, cut to +-clamp); an
+// exact zero would give NaN. Such a parameter is held for this step instead: its
+// row becomes the identity and its gradient zero.
+template <int MODE, int W = 32>
+__device__ __forceinline__ float lm_solve_lanes(int lane, const float (&hr)[ModeTraits<MODE>::NV],
+                                                float gl, bool refine, bool& ok) {
+  constexpr int NV = ModeTraits<MODE>::NV;
+  const int base = (W == 32) ? 0 : (int)(threadIdx.x & 31u & ~(unsigned)(W - 1));
+  bool frz = false;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (lane == k) frz = (hr[k] == 0.0f);
+  const unsigned fmask = __ballot_sync(kFull, frz && lane < NV) >> base;
+  float am[NV], ar[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    am[k] = ((fmask >> k) & 1u) ? 0.0f : hr[k];
+    if (frz) am[k] = (k == lane) ? 1.0f : 0.0f;
+    ar[k] = am[k];
+  }
+  const float rhs = frz ? 0.0f : gl;
+  // Right-looking Cholesky (CPUsplineLib.cpp:1363-1390 computes the same
+  // factor; it fails on a negative pivot only, and what follows is not used).
+  float lr[NV], lc[NV], invd = 1.0f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    lr[j] = 0.0f;
+    lc[j] = 0.0f;
+  }
+  ok = true;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const float ajj = bcast<W>(am[j], j);
+    if (!(ajj >= 0.0f)) ok = false;
+    // 1/sqrt by the hardware reciprocal square root: the refinement step
+    // below absorbs its rounding (the refined steps are unchanged on 3D).
+    const float inv = rsqrtf(ajj);
+    const float ljj = ajj * inv;
+    const float lij = (lane > j) ? am[j] * inv : ((lane == j) ? ljj : 0.0f);
+    lr[j] = lij;
+    if (lane == j) invd = inv;
+#pragma unroll
+    for (int k = j + 1; k < NV; ++k) {
+      const float lkj = bcast<W>(lij, k);
+      if (lane == j) lc[k] = lkj;
+      if (lane > j && k <= lane) am[k] = fmaf(-lij, lkj, am[k]);
+    }
+  }
+  float upd = lane_solve<NV, W>(lane, lr, lc, invd, rhs);
+  if (refine) {
+    // One refinement step: r = b - A upd with error-free products.
+    float sh = rhs, sl = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const float xk = bcast<W>(upd, k);
+      float p_, pe_, t_, te_;
+      two_prod(ar[k], xk, p_, pe_);
+      two_sum(sh, -p_, t_, te_);
+      sh = t_;
+      sl += te_ - pe_;
+    }
+    upd += lane_solve<NV, W>(lane, lr, lc, invd, sh + sl);
+  }
+  if (MODE != 6) {
+    // CPUmleFit_LM.cpp:2943-2950: a NaN step counts as a failed solve
+    constexpr unsigned kRow = (W == 32) ? kFull : (1u << (W & 31)) - 1u;
+    if ((__ballot_sync(kFull, lane < NV && upd != upd) >> base) & kRow) ok = false;
+  }
+  return upd;
+}
+
 // Initial x, y, N, bg of the ROI staged in ws on lanes 0 .. 3 (other lanes 0).
 template <int MODE>
 __device__ __forceinline__ float start_guess(const WarpLayout& L, const float* ws, int lane) {
@@ -1350,17 +1448,17 @@ __device__ __forceinline__ float start_guess(const WarpLayout& L, const float* w
 
 // The fit's first parameters, lane l < NV parameter l: v on lanes 0 .. 3
 // (start_guess), then the start's z, colour, orientation or phase.
-template <int MODE>
-__device__ __forceinline__ float start_params(const FitArgs& a, int lane, int64_t roi, int start,
+template <int MODE, class Args>
+__device__ __forceinline__ float start_params(const Args& a, int lane, int64_t roi, int start,
                                               float v) {
-  if (MODE == 6) {
+  if constexpr (MODE == 6) {
     if (lane == 4) v = (float)a.m.n[2] / 2.0f;
-  } else if (MODE == 7) {
+  } else if constexpr (MODE == 7) {
     const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
     const bool use = (a.n_starts > 0 || a.m.init_p_len >= 2) && ip[0] != 0.0f;
     if (lane == 4) v = use ? ip[0] : (float)a.m.n[2] / 2.0f;
     if (lane == 5) v = use ? ip[1] : (float)a.m.n[3] / 2.0f;
-  } else if (MODE == 8) {
+  } else if constexpr (MODE == 8) {
     // (z, w, u, g2) from initP, shared by all ROIs (CPUmleFit_LM.cpp:3246-3256)
     const float* ip = (a.n_starts > 0) ? a.starts[start] : a.m.init_p;
     if (lane >= 4 && lane < 8) v = ip[lane - 4];
@@ -1476,11 +1574,11 @@ __device__ __forceinline__ float lm_bounds(float par, const ModelDev& m, int s, 
 
 // Takes the step `upd` (lane l < NV: parameter l; fit type 7 scales its colour
 // entry) of a solve that succeeded: clamps, fades and bounds (lm_bounds, or the
-// caller's form of it).
+// caller's form of it). dz: entry 4 of the step (fit type 7). Returns the step
+// that was made, before the bounds; no shuffles, so lanes may stay out.
 template <int MODE, class Bounds>
-__device__ __forceinline__ void lm_apply(LmLane& st, const ModelDev& m, int lane, float& upd,
-                                         Bounds&& bounds) {
-  constexpr int NV = ModeTraits<MODE>::NV;
+__device__ __forceinline__ float lm_apply(LmLane& st, const ModelDev& m, int lane, float& upd, float dz,
+                                          Bounds&& bounds) {
   if (MODE == 7 && lane == 5) upd = upd * 10.0f;  // CPUmleFit_LM.cpp:2951
   st.osg = st.sg;
   st.ocl = st.cl;
@@ -1489,7 +1587,6 @@ __device__ __forceinline__ void lm_apply(LmLane& st, const ModelDev& m, int lane
   st.oerr = st.err;
   if (MODE == 7) {
     // "let it go" (:2966-2971)
-    const float dz = bcast(upd, 4);
     if (fabsf(dz) < 0.005f && st.turn) {
       if (lane == 5) st.cl = st.ocl = (float)m.n[3] / 10.0f;
       if (lane == 4) st.cl = st.ocl = 2.0f;
@@ -1501,8 +1598,18 @@ __device__ __forceinline__ void lm_apply(LmLane& st, const ModelDev& m, int lane
   }
   st.sg = (upd > 0.0f) ? 1.0f : -1.0f;
   const float step = upd / (1.0f + fabsf(upd / st.cl));
-  if (MODE == 8) st.sum_update = warp_sum(lane < NV ? fabsf(step) : 0.0f);
   st.par = bounds(st.par - step);
+  return step;
+}
+
+// Sum of |step| over the parameters, fit type 8's stop quantity. W: lanes of one
+// fit (the levels of a warp's butterfly past them only add zeros).
+template <int NV, int W = 32>
+__device__ __forceinline__ float lm_step_sum(int lane, float step) {
+  float v = lane < NV ? fabsf(step) : 0.0f;
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
 }
 
 // Result of one fit, distributed like the LM state: lane l < NV holds
@@ -1599,80 +1706,13 @@ __device__ RoiResult fit_roi(const FitArgs& a, const WarpLayout& L, float* ws, i
 #pragma unroll
     for (int k = 0; k < NV; ++k)
       if (lane == k) hr[k] *= st.lambda;
-    // A parameter whose derivative is exactly zero at every pixel (z on the
-    // mirror-padded boundary knot) has an exactly zero Hessian row. The
-    // reference only survives that case through rounding noise of its double
-    // derivative sums (a ~1e-29 pivot and a huge step of noise-determined
-    // sign, cut to +-clamp); an exact zero would give NaN. Such a parameter is
-    // held for this step instead: its row becomes the identity and its
-    // gradient zero.
-    bool frz = false;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-      if (lane == k) frz = (hr[k] == 0.0f);
-    const unsigned fmask = __ballot_sync(kFull, frz && lane < NV);
-    float am[NV], ar[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      am[k] = ((fmask >> k) & 1u) ? 0.0f : hr[k];
-      if (frz) am[k] = (k == lane) ? 1.0f : 0.0f;
-      ar[k] = am[k];
-    }
-    const float rhs = frz ? 0.0f : gl;
-    // Right-looking Cholesky (CPUsplineLib.cpp:1363-1390 computes the same
-    // factor; it fails on a negative pivot only).
-    float lr[NV], lc[NV], invd = 1.0f;
     bool ok = true;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      lr[j] = 0.0f;
-      lc[j] = 0.0f;
-    }
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const float ajj = bcast(am[j], j);
-      if (!(ajj >= 0.0f)) {
-        ok = false;
-        break;
-      }
-      // 1/sqrt by the hardware reciprocal square root: the refinement step
-      // below absorbs its rounding (the refined steps are unchanged on 3D).
-      const float inv = rsqrtf(ajj);
-      const float ljj = ajj * inv;
-      const float lij = (lane > j) ? am[j] * inv : ((lane == j) ? ljj : 0.0f);
-      lr[j] = lij;
-      if (lane == j) invd = inv;
-#pragma unroll
-      for (int k = j + 1; k < NV; ++k) {
-        const float lkj = bcast(lij, k);
-        if (lane == j) lc[k] = lkj;
-        if (lane > j && k <= lane) am[k] = fmaf(-lij, lkj, am[k]);
-      }
-    }
-    float upd = 0.0f;
+    float upd = lm_solve_lanes<MODE>(lane, hr, gl, !(a.flags & FLAG_NO_REFINE), ok);
     if (ok) {
-      upd = lane_solve<NV>(lane, lr, lc, invd, rhs);
-      if (!(a.flags & FLAG_NO_REFINE)) {
-        // One refinement step: r = b - A upd with error-free products.
-        float sh = rhs, sl = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-          const float xk = bcast(upd, k);
-          float p_, pe_, t_, te_;
-          two_prod(ar[k], xk, p_, pe_);
-          two_sum(sh, -p_, t_, te_);
-          sh = t_;
-          sl += te_ - pe_;
-        }
-        upd += lane_solve<NV>(lane, lr, lc, invd, sh + sl);
-      }
-      if (MODE != 6) {
-        // CPUmleFit_LM.cpp:2943-2950: a NaN step counts as a failed solve
-        if (__any_sync(kFull, lane < NV && upd != upd)) ok = false;
-      }
-    }
-    if (ok) {
-      lm_apply<MODE>(st, a.m, lane, upd, [&](float p) { return lm_bounds<MODE>(p, a.m, s, lane); });
+      const float dz = (MODE == 7) ? bcast(upd, 4) : 0.0f;
+      const float made = lm_apply<MODE>(st, a.m, lane, upd, dz,
+                                        [&](float p) { return lm_bounds<MODE>(p, a.m, s, lane); });
+      if (MODE == 8) st.sum_update = lm_step_sum<NV>(lane, made);
       need_eval = true;
     } else {
       st.lambda = 10.0f * st.lambda;

@@ -78,6 +78,10 @@ struct FitArgs {
   // launch ends within one ROI's time of its average warp; null: each warp
   // takes every (grid warps)-th ROI. Set by launch_fit.
   unsigned long long* claim;
+  // Slot form only (bsfit_slots.cuh): ROIs in flight per warp at most, and the
+  // number of ROIs left at which a warp with one in flight takes no more.
+  int slots;
+  int64_t spare;
   // Double-float kernels only: per-ROI LM state after the first LM steps of
   // the FP64 reference-order kernel (kHandoffStride doubles per ROI, see
   // Handoff), or null to start from the initial guess.
@@ -135,6 +139,9 @@ struct BatchArgs {
   // higher-priority stream starts as soon as a block's resources free up
   // instead of after the whole launch.
   int warp_rois;
+  // Slot form: as FitArgs
+  int slots;
+  int64_t spare;
   // Work queue in caller-provided device scratch: next[i] is the next
   // unclaimed ROI of segment i, done[i] counts its finished ROIs.
   unsigned long long* next;
@@ -192,6 +199,24 @@ cudaError_t launch_evaldd(const FitArgs& a, const float* theta, double* out, int
                           cudaStream_t stream);
 // Multiprocessors of a device (asked once per process).
 cudaError_t sm_count(int dev, int* sms);
+// A zeroed work counter from the stream-ordered pool, given back to it behind the
+// launch that uses it (on the counter's destruction).
+class WorkCounter {
+ public:
+  unsigned long long* get(cudaStream_t stream);  // null when the pool has none
+  ~WorkCounter();
+
+ private:
+  unsigned long long* p_ = nullptr;
+  cudaStream_t stream_ = nullptr;
+};
+// The fit with several ROIs in flight per warp (fit types 6, 7, 8), where that is
+// the faster form: `warps` is the number that the one-ROI-per-warp form keeps
+// resident, wpb the warps per block (0 to choose). Otherwise *taken stays false and
+// nothing is launched.
+cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, cudaStream_t stream);
+cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, int wpb, int64_t total, int64_t warps,
+                               bool* taken, cudaStream_t stream);
 // Launch shape of a fitter kernel (warps per block among 4, 2, 1 keeping the
 // most warps resident; blocks per SM; SM count), cached per kernel, size and
 // device.
@@ -220,6 +245,7 @@ int tune_rois_per_warp(int mode, int variant);
 int tune_warp_floats(int mode, int variant, int s, bool var);
 FitKern fit_variant(int mode, int variant);     // variant >= 1
 BatchKern batch_variant(int mode, int variant);  // variant >= 1
+BatchKern batch_kern_default(int mode, bool multi, bool cap);
 bool tune_lookup(int mode, int s, int dev, TuneConfig* out);
 bool tune_store(int mode, int s, int dev, TuneConfig c);
 void tune_clear(int mode, int s, int dev);

@@ -1,0 +1,108 @@
+// Launches of the fit kernels with several ROIs in flight per warp
+// (bsfit_slots.cuh).
+#include <cstdint>
+
+#include "bsfit_slots.cuh"
+
+namespace bsfit {
+
+namespace {
+
+template <int MODE>
+FitKern slot_kern_of(bool multi, bool var) {
+  constexpr int B = slot_min_blocks(MODE);
+  if (var) return slot_kernel<MODE, false, true, B>;
+  if constexpr (MODE != 6) {
+    if (multi) return slot_kernel<MODE, true, false, B>;
+  }
+  return slot_kernel<MODE, false, false, B>;
+}
+
+struct SlotLaunch {
+  int slots, per_warp, wpb, bps, sms;
+};
+
+// The slot form's place. Measured on GB300 (ms; one ROI per warp / slot form,
+// W the warps that the first keeps resident):
+//   3D    200,000 x 13 px 5.09 / 4.56    100,000 x 7 px 2.00 / 1.78
+//         50,000 x 21 px 2.73 / 2.69     50,000 x 15 px sCMOS 1.65 / 1.53
+//         batch of 1,000,000 x 11, 13, 17 px 26.9 / 25.0
+//         20,000 x 13 px (5.5 W) 0.593 / 0.561     6,000 (1.6 W) 0.251 / 0.258
+//         batch of 10,000 x 11, 13, 17 px (2.7 W) 0.345 / 0.388
+//   4D    40,000 x 13 px 6.60 / 5.53     20,000 x 17 px 4.72 / 4.27
+//         10,000 x 13 px (4.1 W) 1.87 / 1.75       8,000 x 15 px, 3 starts 5.61 / 5.39
+//   5D    12,000 x 13 px 6.05 / 5.57     8,000 x 17 px 6.75 / 6.70
+//         2,000 x 17 px (1.1 W) 2.16 / 2.34
+// With fewer than three ROIs per warp the slots are seldom full, and the end of the
+// work, several ROIs to a warp, costs more than they save.
+constexpr int64_t kEnough = 3;
+// Warps stop taking further ROIs when two per warp are left: 0, 1, 2, 3 measured
+// 7.54, 7.01, 6.68, 6.77 ms on 8,000 5D ROIs, 5.68, 5.64, 5.54, 5.60 ms on 40,000
+// 4D ROIs, within 0.2% on 200,000 3D ROIs.
+constexpr int64_t kSparePerWarp = 2;
+
+bool enough(int64_t rois, int64_t warps) { return rois >= kEnough * warps; }
+
+// The most slots with which as many warps stay resident as with one ROI per warp
+// (to 5%), or, where the slots' shared memory leaves none, the most that keep 85% of
+// them (21 px 3D ROIs: 17 warps per SM against 20, and still 1.5% faster). q->slots
+// 0: not even two do. more: floats per warp besides the layout's.
+cudaError_t pick_slots(const void* kern, int mode, int s, bool var, bool multi, int more, int wpb,
+                       int64_t warps, SlotLaunch* q) {
+  for (int percent : {95, 85})
+    for (int r = kMaxSlots; r >= 2; --r) {
+      SlotLaunch t{r, (make_slot_layout(mode, s, var, r, multi).total + more) * 4, 0, 0, 0};
+      if (pick_launch_wpb(kern, t.per_warp, wpb, &t.wpb, &t.bps, &t.sms) != cudaSuccess) continue;
+      if ((int64_t)t.wpb * t.bps * t.sms * 100 < percent * warps) continue;
+      *q = t;
+      return cudaSuccess;
+    }
+  return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, cudaStream_t stream) {
+  *taken = false;
+  const bool var = a.var != nullptr, multi = a.n_starts > 1;
+  const int mode = a.m.fittype;
+  if (!enough(a.nfits, warps)) return cudaSuccess;
+  const FitKern kern = mode == 6   ? slot_kern_of<6>(false, var)
+                       : mode == 7 ? slot_kern_of<7>(multi, var)
+                       : mode == 8 ? slot_kern_of<8>(multi, var)
+                                   : nullptr;
+  if (!kern) return cudaSuccess;
+  SlotLaunch q{};
+  const cudaError_t e = pick_slots((const void*)kern, mode, a.s, var, multi, 0, wpb, warps, &q);
+  if (e != cudaSuccess || q.slots < 2) return e;
+  FitArgs b = a;
+  WorkCounter claim;
+  b.slots = q.slots;
+  b.claim = claim.get(stream);
+  if (!b.claim) return cudaSuccess;
+  const int64_t grid = (int64_t)q.sms * q.bps;
+  b.spare = kSparePerWarp * grid * q.wpb;
+  *taken = true;
+  kern<<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, int wpb, int64_t total, int64_t warps,
+                               bool* taken, cudaStream_t stream) {
+  *taken = false;
+  if (!enough(total, warps)) return cudaSuccess;
+  const BatchKern kern = slot_batch_kern(mode, multi);
+  if (!kern) return cudaSuccess;
+  SlotLaunch q{};
+  const cudaError_t e = pick_slots((const void*)kern, mode, a.s_max, false, multi, kSegWords, wpb, warps, &q);
+  if (e != cudaSuccess || q.slots < 2) return e;
+  BatchArgs b = a;
+  b.slots = q.slots;
+  const int64_t grid = (int64_t)q.sms * q.bps;
+  b.spare = kSparePerWarp * grid * q.wpb;
+  *taken = true;
+  kern<<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
+  return cudaGetLastError();
+}
+
+}  // namespace bsfit

@@ -402,7 +402,9 @@ __device__ __forceinline__ RoiResult fit_team(const FitArgs& a, const TeamLayout
         // CPUmleFit_LM.cpp:2943-2950: a NaN step counts as a failed solve
         if (MODE != 6 && nan) ok = false;
         if (ok) {
-          lm_apply<MODE>(st, a.m, lane, upd, [&](float p) { return bounds(p, lane); });
+          const float made =
+              lm_apply<MODE>(st, a.m, lane, upd, x[NV > 4 ? 4 : 0], [&](float p) { return bounds(p, lane); });
+          if (MODE == 8) st.sum_update = lm_step_sum<NV>(lane, made);
           break;
         }
       }

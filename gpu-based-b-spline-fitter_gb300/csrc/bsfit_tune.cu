@@ -17,7 +17,8 @@
 //    that does not grow with the ROI between two ROIs at twice the shared
 //    memory per warp, or both on all 32 lanes in the two halves of paired FP32
 //    operations (bsfit_pack.cuh), which shares the whole evaluation.
-// Variant 0 is the default kernel (bsfit_fit.cu); this file instantiates the
+// Variant 0 is the default: one ROI per warp (bsfit_fit.cu), or several in flight
+// per warp for calls of many ROIs (bsfit_slots.cu); this file instantiates the
 // others. Every variant runs the same code, so results are bit-identical
 // across configurations. A table per (fit type, ROI size, device) holds the
 // chosen configuration; launch_fit and launch_batch consult it.
