@@ -115,9 +115,6 @@ struct ModeTraits<6> {
   static constexpr int NA = 2;   // non-lateral maps: value, d/dz
   static constexpr int NG = 3;   // after the Y pass: value, d/dY, d/dz
   static constexpr int NCH = 1;  // image channels per ROI
-  // stage-B maps written over consumed stage-A columns (see WarpLayout): on
-  // where it lets more warps fit per SM
-  static constexpr bool ALIAS = true;
   // sums reduced over the lanes with the trimmed reduce-scatter (reduce_scatter
   // of the K sums) rather than padded to 32 per exchange tree: a per-model
   // choice by measurement (3D +5%, 4D +1.4%; 5D and 4Pi 1-3% slower)
@@ -130,7 +127,6 @@ struct ModeTraits<7> {
   static constexpr int NA = 3;  // value, d/dz, d/dw
   static constexpr int NG = 4;  // value, d/dY, d/dz, d/dw
   static constexpr int NCH = 1;
-  static constexpr bool ALIAS = true;
   static constexpr bool TRIM_RS = true;
 };
 // 4Pi: the 4D evaluation of fit type 7 once per channel.
@@ -141,7 +137,6 @@ struct ModeTraits<kFit4Pi> {
   static constexpr int NA = 3;
   static constexpr int NG = 4;
   static constexpr int NCH = k4PiChannels;
-  static constexpr bool ALIAS = false;
   static constexpr bool TRIM_RS = false;
 };
 
@@ -157,7 +152,6 @@ struct ModeTraits<8> {
   // d/dY, d/dz (3D)
   static constexpr int NG = 10;
   static constexpr int NCH = 1;
-  static constexpr bool ALIAS = true;
   static constexpr bool TRIM_RS = false;
 };
 
@@ -167,16 +161,16 @@ struct ModeTraits<8> {
 //
 // The stage-A maps (NA per lateral node) and the stage-B maps (NG per X node
 // and pixel row) are both stored by X node ("column"): A column xr holds
-// NA x WP floats, G column xr holds NG x s. For the models whose maps would
-// otherwise bound the warps per SM by shared memory (3D, 4D, 5D), the two share
-// one region: stage B reads only A column xr to write G column xr and walks the
-// columns in order, so G is written over A columns already consumed. With G
-// at the start of the region and A at offset a_rel with
+// NA x WP floats, G column xr holds NG x s. The two share one region, or the
+// maps would bound the warps per SM: stage B reads only A column xr to write G
+// column xr and walks the columns in order, so G is written over A columns
+// already consumed. With G at the start of the region and A at offset a_rel with
 // (xr + 1) * GS <= a_rel + xr * AS for every column, a G column never reaches
 // an A column that is still to be read (the reads and writes of one pass of
-// the warp are separated by __syncwarp). The other models keep the two map
-// sets apart (a_rel = WP * GS) and write G without that synchronisation,
-// which would cost them registers.
+// the warp are separated by __syncwarp). Apart they measured, for 4Pi (8,000 ROIs
+// of 4 x 16 px, 14 warps per SM against 16) 2.54 ms against 2.38, at 24 px 7.61
+// against 6.14. A team's maps are apart (bsfit_team.cuh): all its threads work on
+// one stage at once.
 //
 // Bank-conflict-free access: stage B reads A, and stage C reads G, with s
 // lanes per column in each pass of the warp at the same offsets in every
@@ -235,7 +229,7 @@ __host__ __device__ constexpr WarpLayout make_layout(int mode, int s, bool var =
   L.ng = mode == 6 ? 3 : (mode == 7 || mode == kFit4Pi) ? 4 : 10;
   L.nch = mode == kFit4Pi ? k4PiChannels : 1;
   L.nvar = var ? L.nch : 0;
-  L.alias = mode != kFit4Pi;
+  L.alias = true;
   L.stage = (stg && mode == 8) ? kStageFloats : 0;
   return L;
 }
@@ -265,12 +259,6 @@ constexpr bool layouts_disjoint() {
   return true;
 }
 static_assert(layouts_disjoint(), "per-warp shared-memory regions overlap");
-static_assert(make_layout(6, 13).alias == ModeTraits<6>::ALIAS &&
-                  make_layout(7, 13).alias == ModeTraits<7>::ALIAS &&
-                  make_layout(8, 13).alias == ModeTraits<8>::ALIAS &&
-                  make_layout(kFit4Pi, 13).alias == ModeTraits<kFit4Pi>::ALIAS,
-              "layout aliasing and stage-B synchronisation must agree");
-
 
 // ---------------------------------------------------------------------------
 // One ROI evaluation: deviance, gradient and Hessian (or Fisher information and
@@ -848,7 +836,7 @@ __device__ __forceinline__ void channel_pass(const Args& a, const WarpLayout& L,
         }
       }
       // G aliases A (see WarpLayout; a team's maps do not alias)
-      if constexpr (TR::ALIAS && TW == 0) __syncwarp();
+      if constexpr (TW == 0) __syncwarp();
       if (act) {
         float* go = G + (xr * s + py) * GP;
         if constexpr (MODE == 6) {
