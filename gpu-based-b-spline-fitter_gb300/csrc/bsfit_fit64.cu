@@ -22,16 +22,27 @@
 // the double build it follows. The only other source of difference is the
 // last bit of log().
 //
-// Layout: one warp per ROI. Lanes evaluate pixels 32 at a time and publish
-// each pixel's terms in a shared row (its deviance term, t1 * dudt[l], and
-// (t2 * dudt[l]) * dudt[m], the products the reference adds); the sums are
-// owned one or two entries per lane and accumulated over the rows in pixel
-// order, so every sum has the reference's order. Lane 0 runs the LM control
-// and the small dense solves on shared state. Coefficients are a double copy
-// of the model's table followed by one table per axis of the neighbour
-// differences (-c[i]) + c[i + stride] the derivative terms use (computed once
-// per model, the same double operation). Throughput is bounded by the FP64
-// pipe; this is the parity mode, the FP32 kernels are the production path.
+// Layout: one block of kTeam = 4 warps per ROI: the sums' dependent adds let one
+// warp use a quarter of the SM's FP64 rate, and a call of few ROIs, or the last ones
+// of a large call, lasts as long as one fit. Threads evaluate pixels
+// 128 at a time and publish each pixel's terms in a shared row (its deviance term,
+// t1 * dudt[l], and (t2 * dudt[l]) * dudt[m], the products the reference adds); the
+// sums are owned one per thread and accumulated over the rows in pixel order, so
+// every sum has the reference's order. One warp, another from ROI to ROI so that the
+// four units share it, forms the sums and runs the LM control and the small dense
+// solves, lane l on parameter or row l, on shared state: an FP64 instruction costs
+// the same for one lane as for 32. Coefficients are a double copy of the model's table followed by
+// one table per axis of the neighbour differences (-c[i]) + c[i + stride] the
+// derivative terms use (computed once per model, the same double operation). ROIs are
+// claimed from a work counter when there are more than resident blocks. Throughput
+// is bounded by the FP64 pipe; this is the parity mode, the FP32 kernels are the
+// production path.
+//
+// Measured (GB300, ms; one warp per ROI with the control on one lane / this): one
+// 13 px 3D ROI 1.59 / 0.67, 150 of them 5.34 / 2.20, 3,000 of 11 px 8.93 / 6.63, 20,000
+// of 13 px 64.9 / 55.3 (FP64 pipe 83% / about 82% busy with 16% fewer instructions),
+// 500 4D ROIs of 13 px 40.0 / 34.2, 100 5D ROIs of 17 px 314 / 98 (its weight tables
+// left three warps per SM room, now two blocks of four).
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -46,22 +57,22 @@ template <int MODE>
 struct F64Traits;
 template <>
 struct F64Traits<6> {
-  static constexpr int D = 3, NV = 5, WPB = 4, NCH = 1;
+  static constexpr int D = 3, NV = 5, NCH = 1;
 };
 template <>
 struct F64Traits<7> {
-  static constexpr int D = 4, NV = 6, WPB = 1, NCH = 1;
+  static constexpr int D = 4, NV = 6, NCH = 1;
 };
 template <>
 struct F64Traits<8> {
-  static constexpr int D = 5, NV = 8, WPB = 1, NCH = 1;
+  static constexpr int D = 5, NV = 8, NCH = 1;
 };
 // 4Pi (the restatement in the oracle, oracle/bsfit_oracle.cpp fit_4pi_roi):
 // four channels of the 4D model at theta + dT[c], phase shifted by the
 // channel's shift and wrapped, summed into one likelihood.
 template <>
 struct F64Traits<kFit4Pi> {
-  static constexpr int D = 4, NV = 6, WPB = 1, NCH = k4PiChannels;
+  static constexpr int D = 4, NV = 6, NCH = k4PiChannels;
 };
 
 // Float literals of the reference (VC/CPUmleFit_LM/definitions.h:15, :23-24).
@@ -69,14 +80,17 @@ constexpr float kPIf = 3.141592f;
 constexpr float kTOLf = 1e-6f;
 constexpr float kTOL1f = 1e-5f;
 
-// LM state of one warp, written by lane 0 only (the owners of the sums write
-// err / jac / hes / M / div between two warp barriers).
+constexpr int kTeam = 4, kThreads = 32 * kTeam;
+
+// LM state of one block, written by its lead warp (the owners of the sums write err / jac
+// / hes / M / div between two block barriers).
 struct LMState {
-  double nt[8], ot[8], ns[8], os[8], nc[8], oc[8], fade[8], upd[8], jac[8], diag[8];
-  double hes[64], U[64], M[64], Minv[64];
+  double nt[8], ot[8], ns[8], os[8], nc[8], oc[8], fade[8], jac[8];
+  double hes[64], M[64];
   double newErr, oldErr, newLambda, oldLambda, sumUpdate, div;
   double frame[8];  // yc, xc, off, zc, wc, uc, g2 of the last preparation
-  int turn, action, pad[2];
+  unsigned long long claimed;
+  int turn, action;
 };
 static_assert(sizeof(LMState) % 16 == 0, "LMState keeps the tables 16-byte aligned");
 constexpr int kLMDoubles = (int)(sizeof(LMState) / sizeof(double));
@@ -91,12 +105,12 @@ struct F64Layout {
   static constexpr int AX = 40;                       // 1-D weights, 4 kinds x 5 axes x 2
   static constexpr int NE = 1 + NV + NV * (NV + 1) / 2;  // sums: deviance, gradient, Hessian
   static constexpr int RW = NE;                       // row: one term per sum
-  static constexpr int ROWS = 32 * RW;
+  static constexpr int ROWS = kThreads * RW;
   static constexpr int off_wt = kLMDoubles;
   static constexpr int off_wt3 = off_wt + WT;
   static constexpr int off_ax = off_wt3 + WT3;
   static constexpr int off_rows = off_ax + AX;
-  static constexpr int per_warp = off_rows + ROWS + (ROWS & 1);
+  static constexpr int total = off_rows + ROWS + (ROWS & 1);
 };
 
 // Phase position wrapped into [1, 1 + P), P = nw - 1, by one period.
@@ -162,9 +176,9 @@ __device__ __forceinline__ double axis_weight(double frac, int kind, int v) {
 // (axis a at v = bit a of n, plus 1), b the side bits; the products run over
 // the axes left to right.
 template <int D>
-__device__ __forceinline__ void build_tables(const double* ax, double* W, int lane) {
+__device__ __forceinline__ void build_tables(const double* ax, double* W) {
   constexpr int B = 1 << D, BB = B * B;
-  for (int e = lane; e < BB; e += 32) {
+  for (int e = threadIdx.x; e < BB; e += kThreads) {
     const int n = e >> D, b = e & (B - 1);
     double val[D], der[D];
 #pragma unroll
@@ -266,11 +280,11 @@ struct Fit64Ctx {
   const float* data;  // channel 0's pixels; channel c at data + c * nfits * s * s
   const float* var;
   const float* dT;    // 4Pi: this ROI's [4][6] channel offsets
-  int s, lane;
+  int s;
 };
 
 template <int MODE>
-struct Warp64 {
+struct Team64 {
   using L = F64Layout<MODE>;
   static constexpr int D = L::D, NV = L::NV, RW = L::RW;
   LMState& st;
@@ -278,38 +292,39 @@ struct Warp64 {
   double* wt3;
   double* ax;
   double* rows;
-  // Sum entries owned by this lane (entry t = lane + 32 h, also its index in a
-  // row): kind 0 = deviance / log-likelihood, 1 = gradient l, 2 = Hessian /
-  // Fisher (l, m), m >= l; -1 = none.
-  int kind[2], el[2], em[2];
+  // The sum owned by this thread (entry `own`, also its index in a row): kind 0 =
+  // deviance / log-likelihood, 1 = gradient l, 2 = Hessian / Fisher (l, m), m >= l;
+  // -1 = none.
+  int own = 0, kind = -1, el = 0, em = 0;
 
-  __device__ Warp64(double* base, int lane)
+  __device__ explicit Team64(double* base)
       : st(*reinterpret_cast<LMState*>(base)),
         wt(base + L::off_wt),
         wt3(base + L::off_wt3),
         ax(base + L::off_ax),
-        rows(base + L::off_rows) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int t = lane + 32 * h;
-      kind[h] = -1;
-      el[h] = em[h] = 0;
-      if (t == 0) {
-        kind[h] = 0;
-      } else if (t <= NV) {
-        kind[h] = 1;
-        el[h] = t - 1;
-      } else {
-        int p = t - 1 - NV;
-        for (int l = 0; l < NV; ++l) {
-          if (p < NV - l) {
-            kind[h] = 2;
-            el[h] = l;
-            em[h] = l + p;
-            break;
-          }
-          p -= NV - l;
+        rows(base + L::off_rows) {}
+
+  // The sums go to the threads from warp `lead` on.
+  __device__ void assign(int lead) {
+    static_assert(L::NE <= kThreads, "one sum per thread");
+    const int t = (threadIdx.x - 32 * lead) & (kThreads - 1);
+    own = t;
+    kind = -1;
+    if (t == 0) {
+      kind = 0;
+    } else if (t <= NV) {
+      kind = 1;
+      el = t - 1;
+    } else {
+      int p = t - 1 - NV;
+      for (int l = 0; l < NV; ++l) {
+        if (p < NV - l) {
+          kind = 2;
+          el = l;
+          em = l + p;
+          break;
         }
+        p -= NV - l;
       }
     }
   }
@@ -317,14 +332,13 @@ struct Warp64 {
   // Frame and weight tables at theta (the models' prepare(),
   // CPUmleFit_LM.cpp:2512-2523 and the 4D / 5D copies).
   __device__ void prepare(const Fit64Ctx& cx, const double* th) {
-    const int lane = cx.lane;
     const double half = (double)((cx.s + 1) / 2);
     const double xc = half - th[0], yc = half - th[1];
     const double zc = th[4];
     const double wc = (D >= 4) ? th[5] : 0.0;
     const double uc = (D >= 5) ? th[6] : 0.0;
     double fr[5] = {yc - floor(yc), xc - floor(xc), zc - floor(zc), wc - floor(wc), uc - floor(uc)};
-    for (int t = lane; t < 8 * D; t += 32) {
+    for (int t = threadIdx.x; t < 8 * D; t += kThreads) {
       const int kind = t / (2 * D), r = t - kind * 2 * D, axis = r >> 1, v = (r & 1) + 1;
       double f = fr[0];
 #pragma unroll
@@ -332,7 +346,7 @@ struct Warp64 {
         if (axis == q) f = fr[q];
       ax[(kind * 5 + axis) * 2 + v - 1] = axis_weight(f, kind, v);
     }
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       st.frame[0] = yc;
       st.frame[1] = xc;
       st.frame[3] = zc;
@@ -340,10 +354,10 @@ struct Warp64 {
       st.frame[5] = uc;
       st.frame[6] = (MODE == 8) ? th[7] : 0.0;
     }
-    __syncwarp();
-    build_tables<D>(ax, wt, lane);
-    if constexpr (MODE == 8) build_tables<3>(ax, wt3, lane);
-    __syncwarp();
+    __syncthreads();
+    build_tables<D>(ax, wt);
+    if constexpr (MODE == 8) build_tables<3>(ax, wt3);
+    __syncthreads();
   }
 
   // Value and derivative vector of pixel (ii, jj) with the prepared frame.
@@ -371,17 +385,17 @@ struct Warp64 {
     }
   }
 
-  // The pixels of one plane, in the reference's order (ii outer, jj inner), 32
-  // at a time: each lane publishes its pixel's terms in a row (the deviance
+  // The pixels of one plane, in the reference's order (ii outer, jj inner), 128
+  // at a time: each thread publishes its pixel's terms in a row (the deviance
   // term, t1 * dudt[l] and (t2 * dudt[l]) * dudt[m]; or the log-likelihood term,
   // its use flag and (dudt[m] * dudt[l]) / model), then every owner adds its
   // entry of the rows in pixel order to acc.
   template <bool FISHER>
   __device__ void accumulate_plane(const Fit64Ctx& cx, const float* data, double N, double bg,
-                                   bool dup45, double (&acc)[2]) {
-    const int s = cx.s, s2 = s * s, lane = cx.lane;
-    for (int r0 = 0; r0 < s2; r0 += 32) {
-      const int q = r0 + lane;
+                                   bool dup45, double& acc) {
+    const int s = cx.s, s2 = s * s, me = threadIdx.x;
+    for (int r0 = 0; r0 < s2; r0 += kThreads) {
+      const int q = r0 + me;
       if (q < s2) {
         const int ii = q / s, jj = q - ii * s;
         double dudt[NV], model;
@@ -393,7 +407,7 @@ struct Warp64 {
           model += v;
           dval += v;
         }
-        double* row = rows + lane * RW;
+        double* row = rows + me * RW;
         int k = 1 + NV;
         if constexpr (FISHER) {
           // CPUmleFit_LM.cpp:2730-2742
@@ -431,23 +445,20 @@ struct Warp64 {
           }
         }
       }
-      __syncwarp();
-      const int cnt = (s2 - r0 < 32) ? s2 - r0 : 32;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int kd = kind[h];
-        if (kd < 0 || (FISHER && kd == 1)) continue;
-        const int e = lane + 32 * h;
-        double a = acc[h];
-        if (FISHER && kd == 0) {
+      __syncthreads();
+      const int cnt = (s2 - r0 < kThreads) ? s2 - r0 : kThreads;
+      if (kind >= 0 && !(FISHER && kind == 1)) {
+        double a = acc;
+        if (FISHER && kind == 0) {
           for (int j = 0; j < cnt; ++j)
             if (rows[j * RW + 1] != 0.0) a = a + rows[j * RW];
         } else {
-          for (int j = 0; j < cnt; ++j) a = a + rows[j * RW + e];
+#pragma unroll 8
+          for (int j = 0; j < cnt; ++j) a = a + rows[j * RW + own];
         }
-        acc[h] = a;
+        acc = a;
       }
-      __syncwarp();
+      __syncthreads();
     }
   }
 
@@ -461,7 +472,7 @@ struct Warp64 {
   template <bool FISHER>
   __device__ void pass(const Fit64Ctx& cx, bool dup45) {
     constexpr int NCH = F64Traits<MODE>::NCH;
-    double acc[2] = {0.0, 0.0};
+    double acc = 0.0;
     if constexpr (NCH == 1) {
       accumulate_plane<FISHER>(cx, cx.data, st.nt[2], st.nt[3], dup45, acc);
     } else {
@@ -476,169 +487,170 @@ struct Warp64 {
         accumulate_plane<FISHER>(cx, cx.data + ch * plane, tc[2], tc[3], dup45, acc);
       }
     }
+    if (kind == 0) {
+      if (FISHER) st.div = acc;
+      else st.newErr = acc;
+    } else if (kind == 1) {
+      if (!FISHER) st.jac[el] = acc;
+    } else if (kind == 2) {
+      double* Mx = FISHER ? st.M : st.hes;
+      Mx[el * NV + em] = acc;
+      Mx[em * NV + el] = acc;
+    }
+    __syncthreads();
+  }
+};
+
+__device__ __forceinline__ double shfl64(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// Unpivoted Cholesky (CPUsplineLib.cpp:1363-1390) and the substitutions
+// (:1392-1419) of A x = b on one warp: lane i < NV holds row i of A in h and b_i.
+// Every element is formed by the operations of the reference's loops in their order
+// (the off-diagonal update multiplies by the reciprocal, as written); lanes past NV
+// repeat row NV - 1. Returns 0, or 1 on a negative pivot; x on every lane.
+template <int NV>
+__device__ __forceinline__ int cholesky_solve64(int i, const double (&h)[NV], double b, double (&x)[NV]) {
+  double u[NV], diag = 1.0;  // row i of the factor, U_ii
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int kd = kind[h], l = el[h], mm = em[h];
-      if (kd == 0) {
-        if (FISHER) st.div = acc[h];
-        else st.newErr = acc[h];
-      } else if (kd == 1) {
-        if (!FISHER) st.jac[l] = acc[h];
-      } else if (kd == 2) {
-        double* Mx = FISHER ? st.M : st.hes;
-        Mx[l * NV + mm] = acc[h];
-        Mx[mm * NV + l] = acc[h];
+  for (int j = 0; j < NV; ++j) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < j; ++k) s = s + u[k] * shfl64(u[k], j);
+    const double t = h[j] - s;
+    const double piv = shfl64(t, j);
+    if (!(piv >= 0)) return 1;
+    const double ujj = sqrt(piv);
+    u[j] = (1.0 / ujj) * t;
+    if (i == j) diag = ujj;
+  }
+  double y = b;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const double yj = shfl64(y / diag, j);
+    if (i == j) y = yj;
+    else if (i > j) y = y - u[j] * yj;
+  }
+#pragma unroll
+  for (int r = NV - 1; r >= 0; --r) {
+    double t = shfl64(y, r);
+#pragma unroll
+    for (int j = r + 1; j < NV; ++j) t = t - shfl64(u[r], j) * x[j];
+    x[r] = t / shfl64(diag, r);
+  }
+  return 0;
+}
+
+// LU inverse (MatInvLib.h:17-77, column-major) on one warp: lane c < SZ returns
+// element (c, c). The factorisation column by column, its rows below the diagonal
+// on the lanes; column c of the inverse by lane c.
+template <int SZ>
+__device__ double mat_inv64(double* M, int lane) {
+  for (int jj = 0; jj < SZ; jj++) {
+    if (lane == 0)
+      for (int ii = 1; ii <= jj; ii++) {
+        double t = 0.0;
+        for (int kk = 0; kk <= ii - 1; kk++) t = t + M[ii + kk * SZ] * M[kk + jj * SZ];
+        M[ii + jj * SZ] = M[ii + jj * SZ] - t;
+      }
+    __syncwarp();
+    const int ii = lane;
+    if (ii > jj && ii < SZ) {
+      const double r = 1.0 / M[jj + jj * SZ];
+      if (jj > 0) {
+        double t = 0.0;
+        for (int kk = 0; kk <= jj - 1; kk++) t = t + M[ii + kk * SZ] * M[kk + jj * SZ];
+        M[ii + jj * SZ] = r * (M[ii + jj * SZ] - t);
+      } else {
+        M[ii + jj * SZ] = r * M[ii + jj * SZ];
       }
     }
     __syncwarp();
   }
-};
-
-// Unpivoted Cholesky (CPUsplineLib.cpp:1363-1390), lower factor in U[i*n+j],
-// j <= i; the off-diagonal update multiplies by the reciprocal, as written.
-template <int NV>
-__device__ int cholesky64(const double* A, double* U) {
-  for (int i = 0; i < NV; i++)
-    for (int j = 0; j <= i; j++) {
-      double s = 0.0;
-      for (int k = 0; k < j; k++) s = s + U[i * NV + k] * U[j * NV + k];
-      if (i == j) {
-        if (A[i * NV + i] - s >= 0) U[i * NV + i] = sqrt(A[i * NV + i] - s);
-        else return 1;
-      } else {
-        U[i * NV + j] = (1.0 / U[j * NV + j]) * (A[i * NV + j] - s);
-      }
-    }
-  return 0;
-}
-
-// Forward and backward substitution (CPUsplineLib.cpp:1392-1419).
-template <int NV>
-__device__ void substitute64(const double* U, const double* b, double* x) {
-  double y[NV];
-  for (int i = 0; i < NV; i++) {
-    y[i] = b[i];
-    for (int j = 0; j < i; j++) y[i] = y[i] - U[i * NV + j] * y[j];
-    y[i] = y[i] / U[i * NV + i];
+  const int num = lane < SZ ? lane : SZ - 1;
+  double yy[SZ], inv[SZ], own = 0.0;
+  yy[0] = (num == 0) ? 1.0 : 0.0;
+#pragma unroll
+  for (int ii = 1; ii < SZ; ii++) {
+    const double b = (ii == num) ? 1.0 : 0.0;
+    double t = 0.0;
+#pragma unroll
+    for (int jj = 0; jj <= ii - 1; jj++) t = t + M[ii + jj * SZ] * yy[jj];
+    yy[ii] = b - t;
   }
-  for (int i = NV - 1; i >= 0; i--) {
-    x[i] = y[i];
-    for (int j = i + 1; j < NV; j++) x[i] = x[i] - U[j * NV + i] * x[j];
-    x[i] = x[i] / U[i * NV + i];
+  inv[SZ - 1] = yy[SZ - 1] / M[(SZ - 1) + (SZ - 1) * SZ];
+#pragma unroll
+  for (int ii = SZ - 2; ii >= 0; ii--) {
+    double t = 0.0;
+#pragma unroll
+    for (int jj = ii + 1; jj < SZ; jj++) t = t + M[ii + jj * SZ] * inv[jj];
+    inv[ii] = (1.0 / M[ii + ii * SZ]) * (yy[ii] - t);
   }
-}
-
-// LU inverse returning the diagonal (MatInvLib.h:17-77), column-major.
-template <int SZ>
-__device__ void mat_inv64(double* M, double* Minv, double* diag) {
-  double tmp1 = 0.0;
-  double yy[SZ];
-  for (int jj = 0; jj < SZ; jj++) {
-    for (int ii = 0; ii <= jj; ii++)
-      if (ii > 0) {
-        for (int kk = 0; kk <= ii - 1; kk++) tmp1 = tmp1 + M[ii + kk * SZ] * M[kk + jj * SZ];
-        M[ii + jj * SZ] = M[ii + jj * SZ] - tmp1;
-        tmp1 = 0.0;
-      }
-    for (int ii = jj + 1; ii < SZ; ii++)
-      if (jj > 0) {
-        for (int kk = 0; kk <= jj - 1; kk++) tmp1 = tmp1 + M[ii + kk * SZ] * M[kk + jj * SZ];
-        M[ii + jj * SZ] = (1.0 / M[jj + jj * SZ]) * (M[ii + jj * SZ] - tmp1);
-        tmp1 = 0.0;
-      } else {
-        M[ii + jj * SZ] = (1.0 / M[jj + jj * SZ]) * M[ii + jj * SZ];
-      }
-  }
-  tmp1 = 0.0;
-  for (int num = 0; num < SZ; num++) {
-    yy[0] = (num == 0) ? 1.0 : 0.0;
-    for (int ii = 1; ii < SZ; ii++) {
-      const double b = (ii == num) ? 1.0 : 0.0;
-      for (int jj = 0; jj <= ii - 1; jj++) tmp1 = tmp1 + M[ii + jj * SZ] * yy[jj];
-      yy[ii] = b - tmp1;
-      tmp1 = 0.0;
-    }
-    Minv[SZ - 1 + num * SZ] = yy[SZ - 1] / M[(SZ - 1) + (SZ - 1) * SZ];
-    for (int ii = SZ - 2; ii >= 0; ii--) {
-      for (int jj = ii + 1; jj < SZ; jj++) tmp1 = tmp1 + M[ii + jj * SZ] * Minv[jj + num * SZ];
-      Minv[ii + num * SZ] = (1.0 / M[ii + ii * SZ]) * (yy[ii] - tmp1);
-      tmp1 = 0.0;
-    }
-  }
-  for (int ii = 0; ii < SZ; ii++) diag[ii] = Minv[ii * SZ + ii];
+#pragma unroll
+  for (int ii = 0; ii < SZ; ii++)
+    if (ii == num) own = inv[ii];
+  return own;
 }
 
 // Initial guesses (CPUgaussLib.cpp:172-225, CPUmleFit_LM.cpp:2478-2482,
-// :2839-2850, :3237-3256), lane 0.
-// The single-channel rule on one plane: x, y, N, bg into t[0..3].
-__device__ void guess_plane(const float* d, int s, double* t) {
-  double tx = 0.0, ty = 0.0, ts = 0.0;
+// :2839-2850, :3237-3256), lead warp.
+// The single-channel rule on one plane: x, y, N, bg into t[0..3] on every lane. Lanes
+// 0, 1, 2 sum the moments and the total, lanes 3 and 4 fold the maximum and minimum
+// (of floats, which compare as their doubles do).
+__device__ void guess_plane(const float* d, int s, int lane, double (&t)[4]) {
+  double sum = 0.0;
   for (int ii = 0; ii < s; ii++)
     for (int jj = 0; jj < s; jj++) {
       const double v = (double)d[s * jj + ii];
-      tx = tx + v * (double)ii;
-      ty = ty + v * (double)jj;
-      ts = ts + v;
+      const double w = (lane == 0) ? (double)ii : (double)jj;
+      const double p = v * w;
+      sum = sum + ((lane < 2) ? p : v);
     }
-  t[0] = tx / ts;
-  t[1] = ty / ts;
-  double maxn = 0.0, minbg = (double)10e10f;
-  for (int kk = 0; kk < s; kk++)
-    for (int ll = 0; ll < s; ll++) {
-      const double v = (double)d[kk * s + ll];
-      maxn = (maxn > v) ? maxn : v;
-      minbg = (minbg < v) ? minbg : v;
-    }
+  float fold = (lane == 3) ? 0.0f : 10e10f;
+  for (int p = 0; p < s * s; p++) {
+    const float v = d[p];
+    if (lane == 3) fold = (fold > v) ? fold : v;
+    else fold = (fold < v) ? fold : v;
+  }
+  const double ts = shfl64(sum, 2);
+  const double maxn = (double)__shfl_sync(0xffffffffu, fold, 3), minbg = (double)__shfl_sync(0xffffffffu, fold, 4);
+  t[0] = shfl64(sum, 0) / ts;
+  t[1] = shfl64(sum, 1) / ts;
   const double n0 = ((((maxn - minbg) * 2.0) * (double)kPIf) * 1.5) * 1.5;
   t[2] = (0.0 > n0) ? 0.0 : n0;
   t[3] = (minbg > 0.01) ? minbg : 0.01;
 }
 
+// The first parameters into st.nt.
 template <int MODE>
-__device__ void initial_theta(const Fit64Ctx& cx, LMState& st, int64_t roi) {
+__device__ void initial_theta(const Fit64Ctx& cx, LMState& st, int64_t roi, int lane) {
   constexpr int NV = F64Traits<MODE>::NV;
   const int s = cx.s;
+  double t[4];
   if constexpr (MODE == kFit4Pi) {
     // mean over the channels of the single-channel rule, lateral offsets
     // removed; z and phase per ROI (fit_4pi_roi of the restatement)
     double sx = 0.0, sy = 0.0, sn = 0.0, sb = 0.0;
     for (int c = 0; c < k4PiChannels; ++c) {
-      double t4[4];
-      guess_plane(cx.data + (int64_t)c * cx.a->nfits * s * s, s, t4);
-      sx = sx + (t4[0] - (double)cx.dT[c * NV + 0]);
-      sy = sy + (t4[1] - (double)cx.dT[c * NV + 1]);
-      sn = sn + t4[2];
-      sb = sb + t4[3];
+      guess_plane(cx.data + (int64_t)c * cx.a->nfits * s * s, s, lane, t);
+      sx = sx + (t[0] - (double)cx.dT[c * NV + 0]);
+      sy = sy + (t[1] - (double)cx.dT[c * NV + 1]);
+      sn = sn + t[2];
+      sb = sb + t[3];
     }
-    st.nt[0] = sx / 4.0;
-    st.nt[1] = sy / 4.0;
-    st.nt[2] = sn / 4.0;
-    st.nt[3] = sb / 4.0;
-    st.nt[4] = (double)cx.a->z0[roi];
-    st.nt[5] = wrap_phase64((double)cx.a->w0[roi], cx.a->m.n[3]);
+    if (lane == 0) {
+      st.nt[0] = sx / 4.0;
+      st.nt[1] = sy / 4.0;
+      st.nt[2] = sn / 4.0;
+      st.nt[3] = sb / 4.0;
+      st.nt[4] = (double)cx.a->z0[roi];
+      st.nt[5] = wrap_phase64((double)cx.a->w0[roi], cx.a->m.n[3]);
+    }
     return;
   }
-  const float* d = cx.data;
-  double tx = 0.0, ty = 0.0, ts = 0.0;
-  for (int ii = 0; ii < s; ii++)
-    for (int jj = 0; jj < s; jj++) {
-      const double v = (double)d[s * jj + ii];
-      tx = tx + v * (double)ii;
-      ty = ty + v * (double)jj;
-      ts = ts + v;
-    }
-  st.nt[0] = tx / ts;
-  st.nt[1] = ty / ts;
-  double maxn = 0.0, minbg = (double)10e10f;
-  for (int kk = 0; kk < s; kk++)
-    for (int ll = 0; ll < s; ll++) {
-      const double v = (double)d[kk * s + ll];
-      maxn = (maxn > v) ? maxn : v;
-      minbg = (minbg < v) ? minbg : v;
-    }
-  const double n0 = ((((maxn - minbg) * 2.0) * (double)kPIf) * 1.5) * 1.5;
-  st.nt[2] = (0.0 > n0) ? 0.0 : n0;
-  st.nt[3] = (minbg > 0.01) ? minbg : 0.01;
+  guess_plane(cx.data, s, lane, t);
+  if (lane != 0) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) st.nt[i] = t[i];
   const ModelDev& m = cx.a->m;
   if (MODE == 6) {
     st.nt[4] = (double)m.n[2] / 2.0;
@@ -657,102 +669,119 @@ __device__ __forceinline__ double dmin(double a, double b) { return (a < b) ? a 
 enum { kStop = 0, kEval = 1, kNoEval = 2 };
 
 // One LM iteration up to the evaluation (CPUmleFit_LM.cpp:2569-2640 and the
-// type 7 / 8 copies), lane 0. Returns kStop on convergence, kEval with the new
-// theta in st.nt, or kNoEval after a failed factorization.
+// type 7 / 8 copies), lead warp, lane l < NV on parameter l (lanes past it repeat
+// parameter NV - 1 and write nothing). Returns kStop on convergence, kEval with the
+// new theta in st.nt, or kNoEval after a failed factorization.
 template <int MODE>
-__device__ int lm_control(LMState& st, const ModelDev& m, int s) {
+__device__ int lm_control(LMState& st, const ModelDev& m, int s, int lane) {
   constexpr int NV = F64Traits<MODE>::NV;
-  bool conv = fabs((st.newErr - st.oldErr) / st.newErr) < (double)kTOLf;
+  const int l = lane < NV ? lane : NV - 1;
+  double newErr = st.newErr, oldErr = st.oldErr, newLambda = st.newLambda, oldLambda = st.oldLambda;
+  bool conv = fabs((newErr - oldErr) / newErr) < (double)kTOLf;
   if (MODE == 8) conv = conv || (st.sumUpdate < (double)kTOL1f);
   if (conv) return kStop;
-  if (st.newErr > 1.5 * st.oldErr) {
-    for (int i = 0; i < NV; i++) {
-      st.ns[i] = st.os[i];
-      st.nc[i] = st.oc[i];
-      st.nt[i] = st.ot[i];
-    }
-    st.newLambda = st.oldLambda;
-    st.newErr = st.oldErr;
-    st.newLambda = 10.0 * st.newLambda;
-  } else if (st.newErr < st.oldErr) {
-    if (st.newLambda > 1) st.newLambda = st.newLambda * 0.8;
-    else if (st.newLambda < 1) st.newLambda = 1.0;
+  double ns = st.ns[l], os = st.os[l], nc = st.nc[l], oc = st.oc[l], nt = st.nt[l], ot = st.ot[l];
+  if (newErr > 1.5 * oldErr) {
+    ns = os;
+    nc = oc;
+    nt = ot;
+    newLambda = oldLambda;
+    newErr = oldErr;
+    newLambda = 10.0 * newLambda;
+  } else if (newErr < oldErr) {
+    if (newLambda > 1) newLambda = newLambda * 0.8;
+    else if (newLambda < 1) newLambda = 1.0;
   }
-  for (int i = 0; i < NV; i++) st.hes[i * NV + i] = st.hes[i * NV + i] * st.newLambda;
-  int info = cholesky64<NV>(st.hes, st.U);
-  if (info == 0) {
-    substitute64<NV>(st.U, st.jac, st.upd);
-    if (MODE != 6) {
-      // CPUmleFit_LM.cpp:2943-2950 / :3383-3390
-      for (int l = 0; l < NV; l++)
-        if (isnan(st.upd[l])) info = 1;
-    }
+  double h[NV], x[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    h[k] = st.hes[l * NV + k];
+    if (k == l) h[k] = h[k] * newLambda;
   }
+  const double b = st.jac[l];
+  int turn = st.turn;
+  __syncwarp();  // all reads of the state are done
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (lane == k) st.hes[k * NV + k] = h[k];
+  int info = cholesky_solve64<NV>(l, h, b, x);
+  if (info == 0 && MODE != 6) {
+    // CPUmleFit_LM.cpp:2943-2950 / :3383-3390
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (isnan(x[k])) info = 1;
+  }
+  double sumUpdate = 0.0;
   if (info != 0) {
-    st.newLambda = 10.0 * st.newLambda;
-    return kNoEval;
-  }
-  if (MODE == 7) st.upd[5] = st.upd[5] * 10.0;  // :2951
-  for (int i = 0; i < NV; i++) {
-    st.os[i] = st.ns[i];
-    st.oc[i] = st.nc[i];
-    st.ot[i] = st.nt[i];
-  }
-  st.oldLambda = st.newLambda;
-  st.oldErr = st.newErr;
-  if (MODE == 7) {
-    // "let it go", :2966-2971
-    if (fabs(st.upd[4]) < 0.005 && st.turn) {
-      st.nc[5] = (double)m.n[3] / 10.0;
-      st.oc[5] = st.nc[5];
-      st.turn = 0;
-      st.nc[4] = 2.0;
-      st.oc[4] = 2.0;
+    newLambda = 10.0 * newLambda;
+  } else {
+    if (MODE == 7) x[NV - 1] = x[NV - 1] * 10.0;  // :2951
+    os = ns;
+    oc = nc;
+    ot = nt;
+    oldLambda = newLambda;
+    oldErr = newErr;
+    if (MODE == 7) {
+      // "let it go", :2966-2971
+      if (fabs(x[4]) < 0.005 && turn) {
+        if (l == 5) nc = oc = (double)m.n[3] / 10.0;
+        if (l == 4) nc = oc = 2.0;
+        turn = 0;
+      }
     }
-  }
-  if (MODE == 8) st.sumUpdate = 0.0;
-  for (int ll = 0; ll < NV; ll++) {
-    const double u = st.upd[ll];
-    if (st.ns[ll] != 0) {
-      const bool flip = (st.ns[ll] == 1 && u < 0) || (st.ns[ll] == -1 && u > 0);
-      if (flip) st.nc[ll] = (MODE == 6) ? st.nc[ll] * 0.5 : st.nc[ll] * st.fade[ll];
+    double u = x[0];
+#pragma unroll
+    for (int k = 1; k < NV; ++k)
+      if (l == k) u = x[k];
+    if (ns != 0) {
+      const bool flip = (ns == 1 && u < 0) || (ns == -1 && u > 0);
+      if (flip) nc = (MODE == 6) ? nc * 0.5 : nc * st.fade[l];
     }
-    st.ns[ll] = (u > 0) ? 1.0 : -1.0;
+    ns = (u > 0) ? 1.0 : -1.0;
+    const double v = u / (1.0 + fabs(u / nc));
+    nt = nt - v;
     if (MODE == 8) {
-      const double v = u / (1.0 + fabs(u / st.nc[ll]));
-      st.upd[ll] = v;
-      st.nt[ll] = st.nt[ll] - v;
-      st.sumUpdate = st.sumUpdate + fabs(v);
-    } else {
-      st.nt[ll] = st.nt[ll] - u / (1.0 + fabs(u / st.nc[ll]));
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sumUpdate = sumUpdate + shfl64(fabs(v), k);
+      if (l < 2) {
+        // :3421-3445
+        const double lo = ((double)s - 1.0) / 2.0 - (double)s / 4.0;
+        const double hi = ((double)s - 1.0) / 2.0 + (double)s / 4.0;
+        nt = dmin(dmax(nt, lo), hi);
+      }
+    }
+    if (l == 2) nt = dmax(nt, 1.0);
+    if (l == 3) nt = dmax(nt, 0.01);
+    if (l == 4) nt = dmin(dmax(nt, 0.0), (MODE == 6) ? (double)(m.n[2] - 4) : (double)m.n[2] - 0.5);
+    if (MODE == 7 && l == 5) nt = dmin(dmax(nt, 0.0), (double)m.n[3] - 0.5);
+    if (MODE == kFit4Pi && l == 5) nt = wrap_phase64(nt, m.n[3]);
+    if (MODE == 8) {
+      if (l == 5) {
+        if (nt <= 1) nt = (double)(m.n[3] - 2) + nt;
+        else if (nt > (double)(m.n[3] - 1)) nt = (2.0 + nt) - (double)m.n[3];
+      }
+      if (l == 6) nt = dmin(dmax(nt, 1.0), (double)m.n[4] - 0.5);
+      if (l == 7) nt = dmax(dmin(nt, 1.0), 0.0);
     }
   }
-  if (MODE == 8) {
-    // :3421-3445
-    const double lo = ((double)s - 1.0) / 2.0 - (double)s / 4.0;
-    const double hi = ((double)s - 1.0) / 2.0 + (double)s / 4.0;
-    st.nt[0] = dmin(dmax(st.nt[0], lo), hi);
-    st.nt[1] = dmin(dmax(st.nt[1], lo), hi);
+  if (lane < NV) {
+    st.ns[l] = ns;
+    st.os[l] = os;
+    st.nc[l] = nc;
+    st.oc[l] = oc;
+    st.nt[l] = nt;
+    st.ot[l] = ot;
   }
-  st.nt[2] = dmax(st.nt[2], 1.0);
-  st.nt[3] = dmax(st.nt[3], 0.01);
-  st.nt[4] = dmax(st.nt[4], 0.0);
-  if (MODE == 6) st.nt[4] = dmin(st.nt[4], (double)(m.n[2] - 4));
-  else st.nt[4] = dmin(st.nt[4], (double)m.n[2] - 0.5);
-  if (MODE == 7) {
-    st.nt[5] = dmax(st.nt[5], 0.0);
-    st.nt[5] = dmin(st.nt[5], (double)m.n[3] - 0.5);
+  if (lane == 0) {
+    st.newErr = newErr;
+    st.oldErr = oldErr;
+    st.newLambda = newLambda;
+    st.oldLambda = oldLambda;
+    st.turn = turn;
+    if (MODE == 8 && info == 0) st.sumUpdate = sumUpdate;
   }
-  if (MODE == kFit4Pi) st.nt[5] = wrap_phase64(st.nt[5], m.n[3]);
-  if (MODE == 8) {
-    if (st.nt[5] <= 1) st.nt[5] = (double)(m.n[3] - 2) + st.nt[5];
-    else if (st.nt[5] > (double)(m.n[3] - 1)) st.nt[5] = (2.0 + st.nt[5]) - (double)m.n[3];
-    st.nt[6] = dmax(st.nt[6], 1.0);
-    st.nt[6] = dmin(st.nt[6], (double)m.n[4] - 0.5);
-    st.nt[7] = dmin(st.nt[7], 1.0);
-    st.nt[7] = dmax(st.nt[7], 0.0);
-  }
-  return kEval;
+  __syncwarp();
+  return info != 0 ? kNoEval : kEval;
 }
 
 template <int MODE>
@@ -765,10 +794,9 @@ __device__ void init_state(LMState& st) {
   st.oldErr = 1e13;
   for (int i = 0; i < 8; i++) {
     st.ns[i] = st.os[i] = 0.0;
-    st.upd[i] = 0.0;
     st.jac[i] = 0.0;
   }
-  for (int i = 0; i < 64; i++) st.hes[i] = st.M[i] = st.Minv[i] = st.U[i] = 0.0;
+  for (int i = 0; i < 64; i++) st.hes[i] = st.M[i] = 0.0;
   if (MODE == 6) {
     // :2434
     const double c[5] = {2.0, 2.0, 10000, 20, 20};
@@ -789,36 +817,56 @@ __device__ void init_state(LMState& st) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(32 * F64Traits<MODE>::WPB, 1) fit64_kernel(
-    const __grid_constant__ Fit64Args a) {
+__global__ void __launch_bounds__(kThreads, MODE == 6 ? 4 : MODE == 8 ? 2 : 3) fit64_kernel(const __grid_constant__ Fit64Args a) {
   using L = F64Layout<MODE>;
-  constexpr int NV = L::NV, WPB = F64Traits<MODE>::WPB;
+  constexpr int NV = L::NV;
   extern __shared__ double smem64[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Warp64<MODE> w(smem64 + (int64_t)warp * L::per_warp, lane);
+  const int lane = threadIdx.x & 31;
+  Team64<MODE> w(smem64);
   LMState& st = w.st;
   Fit64Ctx cx;
   cx.a = &a;
   cx.c = Coef{a.c, a.total};
   cx.c3 = Coef{a.c3, a.total3};
   cx.s = a.s;
-  cx.lane = lane;
   const int64_t s2 = (int64_t)a.s * a.s;
-  const int64_t nw = (int64_t)gridDim.x * WPB;
-  for (int64_t roi = (int64_t)blockIdx.x * WPB + warp; roi < a.nfits; roi += nw) {
+  for (int64_t roi = blockIdx.x;; roi += gridDim.x) {
+    if (a.claim) {
+      if (threadIdx.x == 0) st.claimed = atomicAdd(a.claim, 1ull);
+      __syncthreads();
+      roi = (int64_t)st.claimed;
+    }
+    if (roi >= a.nfits) break;
     cx.data = a.rois + roi * s2;
     cx.var = a.var ? a.var + roi * s2 : nullptr;
     cx.dT = (MODE == kFit4Pi) ? a.dT + roi * (int64_t)(k4PiChannels * NV) : nullptr;
-    if (lane == 0) {
-      init_state<MODE>(st);
-      initial_theta<MODE>(cx, st, roi);
-      for (int i = 0; i < NV; i++) {
-        st.ot[i] = st.nt[i];
-        if (MODE == 8) st.oc[i] = st.nc[i];
+    // the warp that does the LM steps and forms the sums, another from ROI to ROI
+    const int lead_warp = (int)(roi & (kTeam - 1));
+    const bool lead = (int)(threadIdx.x >> 5) == lead_warp;
+    w.assign(lead_warp);
+    if (lead) {
+      if (lane == 0) init_state<MODE>(st);
+      initial_theta<MODE>(cx, st, roi, lane);
+      if (lane == 0) {
+        for (int i = 0; i < NV; i++) {
+          st.ot[i] = st.nt[i];
+          if (MODE == 8) st.oc[i] = st.nc[i];
+        }
+        st.frame[2] = (double)((float)(a.m.n[1] - a.s) / 2.0f);  // :2519, float arithmetic
       }
-      st.frame[2] = (double)((float)(a.m.n[1] - a.s) / 2.0f);  // :2519, float arithmetic
     }
-    __syncwarp();
+    __syncthreads();
+    // One LM step by the lead warp, its outcome for everyone.
+    auto control = [&] {
+      if (lead) {
+        const int act = lm_control<MODE>(st, a.m, a.s, lane);
+        if (lane == 0) st.action = act;
+      }
+      __syncthreads();
+      const int act = st.action;
+      __syncthreads();
+      return act;
+    };
     // Initial evaluation; fit type 7 copies dudt[4] into dudt[5] here only.
     // (4Pi prepares per channel inside the pass.)
     if (MODE != kFit4Pi) w.prepare(cx, st.nt);
@@ -828,15 +876,12 @@ __global__ void __launch_bounds__(32 * F64Traits<MODE>::WPB, 1) fit64_kernel(
       // order, then the LM state for the double-float kernels. The step left
       // pending is the last one whose evaluation the double-float kernel makes.
       double te[8];
-      if (lane == 0)
+      if (threadIdx.x == 0)
         for (int i = 0; i < 8; i++) te[i] = st.nt[i];
       int kk = 0, state = Handoff::kCurrent;
       const int K = a.handoff_iters < a.iterations ? a.handoff_iters : a.iterations;
       while (kk < K) {
-        if (lane == 0) st.action = lm_control<MODE>(st, a.m, a.s);
-        __syncwarp();
-        const int act = st.action;
-        __syncwarp();
+        const int act = control();
         if (act == kStop) {
           state = Handoff::kConverged;
           break;
@@ -850,11 +895,11 @@ __global__ void __launch_bounds__(32 * F64Traits<MODE>::WPB, 1) fit64_kernel(
           }
           w.prepare(cx, st.nt);
           w.template pass<false>(cx, false);
-          if (lane == 0)
+          if (threadIdx.x == 0)
             for (int i = 0; i < 8; i++) te[i] = st.nt[i];
         }
       }
-      if (lane == 0) {
+      if (threadIdx.x == 0) {
         double* r = a.handoff + roi * (int64_t)kHandoffStride;
         for (int i = 0; i < 8; i++) {
           const bool in = i < NV;
@@ -877,15 +922,12 @@ __global__ void __launch_bounds__(32 * F64Traits<MODE>::WPB, 1) fit64_kernel(
         r[Handoff::kk] = (double)kk;
         r[Handoff::state] = (double)state;
       }
-      __syncwarp();
+      __syncthreads();
       continue;
     }
     int kk = 0;
     for (; kk < a.iterations; kk++) {
-      if (lane == 0) st.action = lm_control<MODE>(st, a.m, a.s);
-      __syncwarp();
-      const int act = st.action;
-      __syncwarp();
+      const int act = control();
       if (act == kStop) break;
       if (act == kEval) {
         if (MODE != kFit4Pi) w.prepare(cx, st.nt);
@@ -897,17 +939,19 @@ __global__ void __launch_bounds__(32 * F64Traits<MODE>::WPB, 1) fit64_kernel(
     // (CPUmleFit_LM.cpp:3568-3584).
     if (MODE != 8 && MODE != kFit4Pi) w.prepare(cx, st.nt);
     w.template pass<true>(cx, false);
-    if (lane == 0) {
-      mat_inv64<NV>(st.M, st.Minv, st.diag);
+    if (lead) {
+      const double var = mat_inv64<NV>(st.M, lane);
       const int64_t n = a.nfits;
-      for (int i = 0; i < NV; i++) {
-        a.P[n * i + roi] = st.nt[i];
-        a.CRLB[n * i + roi] = st.diag[i];
+      if (lane < NV) {
+        a.P[n * lane + roi] = st.nt[lane];
+        a.CRLB[n * lane + roi] = var;
       }
-      a.P[n * NV + roi] = (double)kk;
-      a.LL[roi] = st.div;
+      if (lane == 0) {
+        a.P[n * NV + roi] = (double)kk;
+        a.LL[roi] = st.div;
+      }
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -941,8 +985,7 @@ std::mutex g_launch64_mu;
 template <int MODE>
 cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
   using L = F64Layout<MODE>;
-  constexpr int WPB = F64Traits<MODE>::WPB;
-  const size_t smem = (size_t)L::per_warp * WPB * sizeof(double);
+  const size_t smem = (size_t)L::total * sizeof(double);
   static Launch64 cache[8];  // per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -957,7 +1000,7 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
                                (int)smem);
       if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev);
       if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.per_sm, fit64_kernel<MODE>, 32 * WPB,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.per_sm, fit64_kernel<MODE>, kThreads,
                                                           smem);
       if (e != cudaSuccess) return e;
       c.dev = dev;
@@ -966,10 +1009,12 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
     sms = c.sms;
   }
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const int64_t need = (a.nfits + WPB - 1) / WPB;
   const int64_t cap = (int64_t)sms * per_sm;
-  const int grid = (int)(need < cap ? need : cap);
-  fit64_kernel<MODE><<<grid, 32 * WPB, smem, stream>>>(a);
+  const int64_t grid = a.nfits < cap ? a.nfits : cap;
+  Fit64Args b = a;
+  WorkCounter claim;
+  if (a.nfits > grid) b.claim = claim.get(stream);
+  fit64_kernel<MODE><<<(unsigned)grid, kThreads, smem, stream>>>(b);
   return cudaGetLastError();
 }
 
@@ -977,10 +1022,10 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
 
 int fit64_smem_bytes(int mode) {
   switch (mode) {
-    case 6: return F64Layout<6>::per_warp * F64Traits<6>::WPB * 8;
-    case 7: return F64Layout<7>::per_warp * F64Traits<7>::WPB * 8;
-    case 8: return F64Layout<8>::per_warp * F64Traits<8>::WPB * 8;
-    case kFit4Pi: return F64Layout<kFit4Pi>::per_warp * F64Traits<kFit4Pi>::WPB * 8;
+    case 6: return F64Layout<6>::total * 8;
+    case 7: return F64Layout<7>::total * 8;
+    case 8: return F64Layout<8>::total * 8;
+    case kFit4Pi: return F64Layout<kFit4Pi>::total * 8;
     default: return 0;
   }
 }

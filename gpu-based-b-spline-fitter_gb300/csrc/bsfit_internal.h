@@ -177,6 +177,8 @@ struct Fit64Args {
   // (kHandoffStride doubles per ROI) instead of outputs.
   double* handoff;
   int handoff_iters;
+  // Work counter (zeroed), or null: each warp takes every (grid warps)-th ROI.
+  unsigned long long* claim;
 };
 
 cudaError_t launch_fit64(const Fit64Args& a, cudaStream_t stream);
