@@ -19,9 +19,9 @@
 // the same butterfly tree; the LM step is the lane-parallel one's operations in
 // its order (lm_solve).
 //
-// Measured (GB300): one 13 px 3D ROI 30.8 us per call against 54.3 us with one
-// warp, 300 of them 58.3 against 99.5 us; where each form is used and what it
-// measured there: bsfit_team.cu.
+// Measured (GB300): one 13 px 3D ROI 28 us per call against 54 us with one warp, 300
+// of them 53 against 99 us; where each form is used and what it measured there:
+// bsfit_team.cu.
 #pragma once
 
 #include "bsfit_fit_kernels.cuh"
@@ -478,14 +478,12 @@ __global__ void __launch_bounds__(32 * T, MINB) team_kernel(const __grid_constan
   fit_and_store_team<MODE, MULTI, VAR, T>(a, TL, reinterpret_cast<float*>(smem4), (int64_t)blockIdx.x);
 }
 
-// The kernel of T warps for a fit type (null: that form is not built). Resident
-// blocks per SM: as many as leave 64 (3D) or 128 registers per thread.
+// The kernel of T warps for a fit type, compiled for B resident blocks per SM.
 using TeamKern = void (*)(const FitArgs);
 constexpr int kTeamMaxShared = 227 * 1024;
 
-template <int MODE, int T>
-TeamKern team_kern_of(bool multi, bool var) {
-  constexpr int B = T == 16 ? 1 : (MODE == 6 ? 4 : 2) * (8 / T);
+template <int MODE, int T, int B>
+TeamKern team_kern(bool multi, bool var) {
   if constexpr (MODE != kFit4Pi) {
     if (var) return team_kernel<MODE, false, true, T, B>;
   }
@@ -495,23 +493,9 @@ TeamKern team_kern_of(bool multi, bool var) {
   return team_kernel<MODE, false, false, T, B>;
 }
 
-template <int T>
-TeamKern team_kern(int mode, bool multi, bool var) {
-  switch (mode) {
-    case 6:
-      if constexpr (T <= 8) return team_kern_of<6, T>(multi, var);
-      else return nullptr;
-    case 7:
-      if constexpr (T <= 8) return team_kern_of<7, T>(multi, var);
-      else return nullptr;
-    case 8: return team_kern_of<8, T>(multi, var);
-    case kFit4Pi: return team_kern_of<kFit4Pi, T>(multi, var);
-    default: return nullptr;
-  }
-}
-
-TeamKern team_kern4(int mode, bool multi, bool var);
-TeamKern team_kern8(int mode, bool multi, bool var);
+// The kernels are compiled in several files; each returns null for what it lacks.
+TeamKern team_kern4(int mode, int blocks, bool multi, bool var);
+TeamKern team_kern4_dense(int mode, int blocks, bool multi, bool var);
 TeamKern team_kern16(int mode, bool multi, bool var);
 
 }  // namespace bsfit

@@ -67,7 +67,7 @@ def test_block_form_is_bit_identical(bsfit_mod, fittype, s):
         for its in ((0, 1, 30) if kind == "plain" else (12,)):
             r, e = pick(many)
             ref = [x.cpu().numpy()[..., :] for x in _call(bsfit_mod, fittype, r, its, model, e, kind)]
-            for n in (1, 150, 300, 600):
+            for n in (1, 150, 300, 400, 600, 740, 900):
                 r, e = pick(many[:n])
                 out = [x.cpu().numpy() for x in _call(bsfit_mod, fittype, r, its, model, e, kind)]
                 for a, b in zip(out, ref):
