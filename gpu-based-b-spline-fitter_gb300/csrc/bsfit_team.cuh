@@ -267,8 +267,9 @@ __device__ __forceinline__ bool lm_solve(const float* S, int lane, const int (&r
 #pragma unroll
   for (int i = 0; i < NV; ++i) rb[i] = bcast(r, i);
   chol_substitute<NV>(l, invd, rb, dx);
+  // (rounded apart: contracted with dx[0]'s product it differs from the lanes' sum)
 #pragma unroll
-  for (int i = 0; i < NV; ++i) x[i] += dx[i];
+  for (int i = 0; i < NV; ++i) x[i] = __fadd_rn(x[i], dx[i]);
   return true;
 }
 

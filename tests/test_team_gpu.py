@@ -73,3 +73,20 @@ def test_block_form_is_bit_identical(bsfit_mod, fittype, s):
                 for a, b in zip(out, ref):
                     assert np.array_equal(a, b[..., :n], equal_nan=True), (kind, its, n)
     model.close()
+
+
+def test_ill_conditioned_solve_rounds_alike(bsfit_mod):
+    """5D fits of 5 px ROIs: the refinement of their nearly singular steps is large
+    enough that a contracted sum would show."""
+    import torch
+    from bsfit import workloads as W
+    w = W.workload_5d(24000, s=5, stream=5)
+    model = bsfit_mod.Model(8, w.coeff, coeff3=w.coeff3, init_p=w.init_p)
+    r = torch.from_numpy(np.ascontiguousarray(w.rois)).cuda()
+    ref = [x.cpu().numpy() for x in model.fit_torch(r, 3)]
+    for n in (150, 300, 450, 600, 750):
+        parts = [model.fit_torch(r[i:i + n].contiguous(), 3) for i in range(0, len(r) - n + 1, n)]
+        for k, b in enumerate(ref):
+            a = np.concatenate([p[k].cpu().numpy() for p in parts], axis=-1)
+            assert np.array_equal(a, b[..., :a.shape[-1]], equal_nan=True), (n, k)
+    model.close()
