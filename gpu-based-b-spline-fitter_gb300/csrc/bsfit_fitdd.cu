@@ -1027,7 +1027,11 @@ __device__ __forceinline__ dd from_double(double v) {
   return dd{h, __double2float_rn(v - (double)h)};
 }
 
-template <int MODE>
+// The warps of a block start every evaluation together (see fitdd_kernel). False
+// when no warp of the block has a fit left.
+__device__ __forceinline__ bool keep_step(bool fitting) { return __syncthreads_or(fitting); }
+
+template <int MODE, bool STEP>
 __device__ Result fit_roi(const FitArgs& a, const Layout& L, float* ws, int lane, int64_t roi) {
   using TR = Traits<MODE>;
   constexpr int NV = TR::NV;
@@ -1116,6 +1120,7 @@ __device__ Result fit_roi(const FitArgs& a, const Layout& L, float* ws, int lane
       for (int k = 0; k < NV; ++k)
         the[k] = shfl((MODE == 8 && fisher && k != 2 && k != 3) ? par_eval : par, k);
       dd e;
+      if (STEP) keep_step(true);
       evaluate<MODE>(a, L, ws, lane, the, first && MODE == 7, fisher, e, gl, hr, maps_ready);
       first = false;
       need_eval = false;
@@ -1341,11 +1346,25 @@ __device__ Result fit_roi(const FitArgs& a, const Layout& L, float* ws, int lane
   return Result{to_f(par), crlb, to_f(ll), kk};
 }
 
-// Minimum resident 4-warp blocks per SM: 3D fits in 128 registers (16 warps per
-// SM, 4 bytes of spill); 4D and 5D keep their register need (167 and 255; a
-// 128-register cap spills 0.5 and 1.5 KB per thread).
+// One warp per ROI, one block per SM. What bounds it is the instruction supply: an
+// evaluation runs some 10,000 double-float instructions of mostly straight-line
+// code, far more than the instruction caches hold, so warps at different places of
+// it evict each other's lines (16 independent warps per SM: 5.4 of 9.4 cycles per
+// instruction were waits for an instruction). With STEP all warps of the block
+// start each evaluation together (keep_step) and share the lines: 0.23 of 6.7
+// cycles, 1.2 of them at the barrier. Measured (GB300, us per call, independent /
+// in step): 3D 13 px 10,000 ROIs 2,108 / 1,485, 40,000 8,200 / 5,274; 3D 21 px
+// 10,000 4,680 / 3,430; 4D 13 px 24,950 / 18,690; 5D 13 px 74,000 / 36,120. Blocks
+// of 4 and 8 warps in step, several per SM: 3D 13 px 2,010 and 1,684.
+// Every warp reaches the barrier before each of its evaluations and, out of ROIs,
+// until the block's last fit ends, so the arrivals match.
+// Warps per block: what the register file holds (3D 128 registers, 4D 168, 5D 255;
+// a 128-register cap spills 0.5 and 1.5 KB per thread in 4D and 5D).
 template <int MODE>
-__global__ void __launch_bounds__(128, MODE == 6 ? 4 : 1) fitdd_kernel(FitArgs a) {
+constexpr int kMaxWarps = MODE == 6 ? 16 : MODE == 7 ? 12 : 8;
+
+template <int MODE, bool STEP>
+__global__ void __launch_bounds__(STEP ? 32 * kMaxWarps<MODE> : 128, STEP ? 1 : 4) fitdd_kernel(FitArgs a) {
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   constexpr int NV = Traits<MODE>::NV;
@@ -1367,7 +1386,7 @@ __global__ void __launch_bounds__(128, MODE == 6 ? 4 : 1) fitdd_kernel(FitArgs a
     const float* src = a.rois + roi * (int64_t)s2;
     for (int p = lane; p < s2; p += 32) ws[p] = __ldg(src + p);
     __syncwarp();
-    const Result r = fit_roi<MODE>(a, L, ws, lane, roi);
+    const Result r = fit_roi<MODE, STEP>(a, L, ws, lane, roi);
     float thv[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) thv[k] = __shfl_sync(kFull, r.par, k);
@@ -1381,6 +1400,8 @@ __global__ void __launch_bounds__(128, MODE == 6 ? 4 : 1) fitdd_kernel(FitArgs a
     if (lane < NV) a.CRLB[lane * n + o] = r.crlb;
     __syncwarp();
     if (!a.claim) roi += total_warps;
+  }
+  while (STEP && keep_step(false)) {
   }
 }
 
@@ -1425,6 +1446,9 @@ __global__ void __launch_bounds__(128) evaldd_kernel(FitArgs a, const float* the
 
 }  // namespace ddf
 
+constexpr int kMaxShared = 227 * 1024;  // bytes per block
+constexpr int kAlone3D = 7;             // ROIs per SM of a 3D call that are fitted uncoupled
+
 int fitdd_smem_floats(int mode, int s) { return ddf::make_layout(mode, s).total(); }
 
 cudaError_t launch_evaldd(const FitArgs& a, const float* theta, double* out, int fisher,
@@ -1451,13 +1475,33 @@ cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream) {
   if (a.nfits <= 0) return cudaSuccess;
   const int mode = a.m.fittype;
   void (*kern)(FitArgs) = nullptr;
-  if (mode == 6) kern = ddf::fitdd_kernel<6>;
-  else if (mode == 7) kern = ddf::fitdd_kernel<7>;
-  else if (mode == 8) kern = ddf::fitdd_kernel<8>;
+  int most = 0;
+  if (mode == 6) kern = ddf::fitdd_kernel<6, true>, most = ddf::kMaxWarps<6>;
+  else if (mode == 7) kern = ddf::fitdd_kernel<7, true>, most = ddf::kMaxWarps<7>;
+  else if (mode == 8) kern = ddf::fitdd_kernel<8, true>, most = ddf::kMaxWarps<8>;
   else return cudaErrorInvalidValue;
-  const int per_warp = fitdd_smem_floats(mode, a.s) * 4;
-  int wpb = 4, bps = 0, sms = 0;
-  cudaError_t e = pick_launch((const void*)kern, per_warp, &wpb, &bps, &sms);
+  const int per_warp = (fitdd_smem_floats(mode, a.s) * 4 + 15) & ~15;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = sm_count(dev, &sms);
+  if (e != cudaSuccess) return e;
+  // Whole quads, so that every scheduler has the same number of warps (us, 10,000
+  // ROIs: 3D 21 px 9 warps 3,691, 8 warps 3,428; 5D 17 px 7 warps 82,100, 4 77,900).
+  if (most > kMaxShared / per_warp) most = kMaxShared / per_warp;
+  if (most > 4) most &= ~3;
+  // 3D fits that leave the SMs nearly empty run uncoupled in blocks of 4: few warps
+  // compete for the instruction cache, and in step they wait for the slowest (us,
+  // coupled / uncoupled, 7 px: 600 ROIs 317 / 298, 1,000 376 / 311, 1,700 407 / 403;
+  // 13 px: 285 / 272, 336 / 318, 407 / 430; 21 px, 1,300 ROIs 688 / 829). For 4D and
+  // 5D in step is as fast or faster from the start (5D, 800 ROIs 5,301 / 6,669).
+  const bool in_step = mode != 6 || a.nfits > (int64_t)kAlone3D * sms;
+  if (!in_step) {
+    kern = ddf::fitdd_kernel<6, false>;
+    if (most > 4) most = 4;
+  }
+  const int64_t each = in_step ? (a.nfits + sms - 1) / sms : most;
+  int wpb = each < most ? (int)each : most < 1 ? 1 : most, bps = 0;
+  e = pick_launch_wpb((const void*)kern, per_warp, wpb, &wpb, &bps, &sms);
   if (e != cudaSuccess) return e;
   const int smem = per_warp * wpb;
   int64_t need = (a.nfits + wpb - 1) / wpb;
