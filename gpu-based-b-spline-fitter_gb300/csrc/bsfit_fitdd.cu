@@ -1447,7 +1447,8 @@ __global__ void __launch_bounds__(128) evaldd_kernel(FitArgs a, const float* the
 }  // namespace ddf
 
 constexpr int kMaxShared = 227 * 1024;  // bytes per block
-constexpr int kAlone3D = 7;             // ROIs per SM of a 3D call that are fitted uncoupled
+constexpr int kAlone3D = 7;             // most ROIs per SM of a 3D call fitted on their own
+constexpr int kInStep3D = 8;            // fewest warps per SM for 3D fits in step
 
 int fitdd_smem_floats(int mode, int s) { return ddf::make_layout(mode, s).total(); }
 
@@ -1485,23 +1486,26 @@ cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = sm_count(dev, &sms);
   if (e != cudaSuccess) return e;
-  // Whole quads, so that every scheduler has the same number of warps (us, 10,000
-  // ROIs: 3D 21 px 9 warps 3,691, 8 warps 3,428; 5D 17 px 7 warps 82,100, 4 77,900).
   if (most > kMaxShared / per_warp) most = kMaxShared / per_warp;
-  if (most > 4) most &= ~3;
-  // 3D fits that leave the SMs nearly empty run uncoupled in blocks of 4: few warps
-  // compete for the instruction cache, and in step they wait for the slowest (us,
-  // coupled / uncoupled, 7 px: 600 ROIs 317 / 298, 1,000 376 / 311, 1,700 407 / 403;
-  // 13 px: 285 / 272, 336 / 318, 407 / 430; 21 px, 1,300 ROIs 688 / 829). For 4D and
-  // 5D in step is as fast or faster from the start (5D, 800 ROIs 5,301 / 6,669).
-  const bool in_step = mode != 6 || a.nfits > (int64_t)kAlone3D * sms;
-  if (!in_step) {
+  // 3D fits that leave the SMs nearly empty, or of which few fit an SM's shared memory,
+  // run on their own in small blocks: few warps compete for the instruction cache, and
+  // in step they wait for the slowest (us, in step / on their own; 7 px: 600 ROIs
+  // 317 / 298, 1,000 376 / 311, 1,700 407 / 403; 13 px: 285 / 272, 336 / 318,
+  // 407 / 430; 21 px, 1,300 ROIs 688 / 829; 4,000 ROIs, four iterations: 23 px, 7 warps
+  // per SM, 1,002 / 992, 27 px, 6 warps, 1,774 / 1,520). For 4D and 5D in step is as
+  // fast or faster from the start (5D, 800 ROIs 5,301 / 6,669).
+  int wpb = 4, bps = 0;
+  if (mode == 6 && (most < kInStep3D || a.nfits <= (int64_t)kAlone3D * sms)) {
     kern = ddf::fitdd_kernel<6, false>;
-    if (most > 4) most = 4;
+    e = pick_launch((const void*)kern, per_warp, &wpb, &bps, &sms);
+  } else {
+    // Whole quads, so that every scheduler has the same number of warps (10,000 ROIs:
+    // 3D 21 px 9 warps 3,691 us, 8 warps 3,428; 5D 17 px 7 warps 82,100, 4 77,900).
+    if (most > 4) most &= ~3;
+    const int64_t each = (a.nfits + sms - 1) / sms;
+    wpb = each < most ? (int)each : most < 1 ? 1 : most;
+    e = pick_launch_wpb((const void*)kern, per_warp, wpb, &wpb, &bps, &sms);
   }
-  const int64_t each = in_step ? (a.nfits + sms - 1) / sms : most;
-  int wpb = each < most ? (int)each : most < 1 ? 1 : most, bps = 0;
-  e = pick_launch_wpb((const void*)kern, per_warp, wpb, &wpb, &bps, &sms);
   if (e != cudaSuccess) return e;
   const int smem = per_warp * wpb;
   int64_t need = (a.nfits + wpb - 1) / wpb;
