@@ -525,7 +525,11 @@ int multid_call(const float* imstack, int64_t roi_size, int64_t roi_size2, int64
   // land, so chunk i + 1 uploads while chunk i fits and the tail of one fit
   // launch overlaps the start of the next. The first chunk is small, so the
   // first fit starts after a short upload, and the chunks double from there
-  // (uploads run several times faster than fits, so they stay ahead). Each
+  // (uploads run several times faster than fits, so they stay ahead). A last
+  // chunk under a quarter of its size is fitted with the one before: its upload
+  // costs less than the tail of one more fit launch (us per call, apart / with
+  // it: 13 px, 20,000 ROIs 758 / 730, 60,000 1,786 / 1,660; 7 px, 18,000 607 / 557;
+  // 21 px, 60,000 3,628 / 3,497). Each
   // chunk's results go back to the host as soon as its fit ends, one strided
   // copy per output (the outputs are column-major over all ROIs), so only the
   // last chunk's copy remains after the last fit. Device buffers come from the
@@ -542,6 +546,7 @@ int multid_call(const float* imstack, int64_t roi_size, int64_t roi_size2, int64
       cb[nchunk++] = b;
       b += c;
       c *= 2;
+      if (nfits - b < c / 4) b = nfits;
     }
     cb[nchunk] = nfits;
   }
