@@ -895,7 +895,7 @@ def bench_gpu(args):
             # throughput: the fraction of the SM's issue rate it sustains.
             issue = {"ipc": prof["ipc"], "max_ipc": prof["max_ipc"],
                      "frac": prof["ipc"] / prof["max_ipc"],
-                     "source": "ncu, profiles/batch_kernel_3d_200k.md"}
+                     "source": "ncu, profiles/slot_batch_kernel_3d_200k.md"}
         except Exception:
             traffic = None
     line = {
