@@ -36,12 +36,18 @@ struct SlotLaunch {
 // With fewer than three ROIs per warp the slots are seldom full, and the end of the
 // work, several ROIs to a warp, costs more than they save.
 constexpr int64_t kEnough = 3;
+// A 3D batch shares its warps among ROI sizes in the order of their cost, and its
+// slots (sized for the largest) are drained at each change. Measured, us, one ROI
+// per warp / slots: 11, 13, 17 px 11,500 ROIs (3.2 W) 380 / 421, 20,000 619 / 657,
+// 36,000 (9.9 W) 1,048 / 1,072, 45,000 (12.3 W) 1,313 / 1,319, 60,000 1,715 / 1,684;
+// 13 px alone 15,000 444 / 457, 20,000 570 / 567, 30,000 806 / 793. 4D 13, 15 px 9,500
+// (3.9 W) 1,891 / 1,876, 20,000 3,655 / 3,575; 5D 17 px 5,600 5,041 / 5,035, 14,000
+// 11,671 / 11,548.
+constexpr int64_t kEnoughBatch3D = 12;
 // Warps stop taking further ROIs when two per warp are left: 0, 1, 2, 3 measured
 // 7.54, 7.01, 6.68, 6.77 ms on 8,000 5D ROIs, 5.68, 5.64, 5.54, 5.60 ms on 40,000
 // 4D ROIs, within 0.2% on 200,000 3D ROIs.
 constexpr int64_t kSparePerWarp = 2;
-
-bool enough(int64_t rois, int64_t warps) { return rois >= kEnough * warps; }
 
 // The most slots with which as many warps stay resident as with one ROI per warp
 // (to 5%), or, where the slots' shared memory leaves none, the most that keep 85% of
@@ -66,7 +72,7 @@ cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, 
   *taken = false;
   const bool var = a.var != nullptr, multi = a.n_starts > 1;
   const int mode = a.m.fittype;
-  if (!enough(a.nfits, warps)) return cudaSuccess;
+  if (a.nfits < kEnough * warps) return cudaSuccess;
   const FitKern kern = mode == 6   ? slot_kern_of<6>(false, var)
                        : mode == 7 ? slot_kern_of<7>(multi, var)
                        : mode == 8 ? slot_kern_of<8>(multi, var)
@@ -90,7 +96,7 @@ cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, 
 cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, int wpb, int64_t total, int64_t warps,
                                bool* taken, cudaStream_t stream) {
   *taken = false;
-  if (!enough(total, warps)) return cudaSuccess;
+  if (total < (mode == 6 ? kEnoughBatch3D : kEnough) * warps) return cudaSuccess;
   const BatchKern kern = slot_batch_kern(mode, multi);
   if (!kern) return cudaSuccess;
   SlotLaunch q{};

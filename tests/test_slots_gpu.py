@@ -49,7 +49,7 @@ def test_many_rois_equal_few(bsfit_mod, fittype, s):
     rois, model, starts = _setup(bsfit_mod, fittype, s)
     rois = _spoil(rois)
     n = len(rois)
-    big = BIG if fittype == 6 else 9000 if fittype == 7 else 6000
+    big = 40000 if fittype == 6 else 9000 if fittype == 7 else 6000
     many = np.random.default_rng(s).integers(0, n, big)
     few = torch.from_numpy(rois).cuda()
     lots = few[torch.from_numpy(many).cuda()].contiguous()
@@ -72,7 +72,7 @@ def test_batches_equal_few(bsfit_mod, fittype, sizes, several):
     if several and fittype == 6:
         pytest.skip("fit type 6 has one start")
     parts, entries, first = [], [], None
-    big = BIG if fittype == 6 else 9000 if fittype == 7 else 6000
+    big = 40000 if fittype == 6 else 9000 if fittype == 7 else 6000
     for k, s in enumerate(sizes + sizes[:1]):
         rois, model, starts = _setup(bsfit_mod, fittype, s)
         first = first or starts
