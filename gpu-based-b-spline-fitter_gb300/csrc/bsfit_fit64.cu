@@ -1014,9 +1014,15 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int64_t cap = (int64_t)sms * per_sm;
   const int64_t grid = a.nfits < cap ? a.nfits : cap;
+  // More ROIs than resident blocks: claimed one at a time, but from fixed shares in a
+  // capture, which then records the launch alone (a graph with the counter's memory
+  // nodes could not be a child of another, nor be cloned).
   Fit64Args b = a;
   WorkCounter claim;
-  if (a.nfits > grid) b.claim = claim.get(stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (a.nfits > grid && cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
+      capture == cudaStreamCaptureStatusNone)
+    b.claim = claim.get(stream);
   fit64_kernel<MODE><<<(unsigned)grid, kThreads, smem, stream>>>(b);
   return cudaGetLastError();
 }
