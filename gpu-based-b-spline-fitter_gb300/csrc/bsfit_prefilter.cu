@@ -65,15 +65,20 @@ __device__ __forceinline__ void filter_line(double* x, int n, int step, const Fi
   double y = y0;
   x[0] = y0;
 #pragma unroll 4
-  for (int k = 1; k < n; ++k) {
+  for (int k = 1; k < n - 1; ++k) {
     y = x[k * step] + z * y;
     x[k * step] = y;
   }
+  y = x_last + z * y;
   y = (2.0 * y - x_last) * fc.c0;
+  // each element is read one step ahead of its use: put may write to the line
+  double next = x[(n - 2) * step];
   put(n - 1, y * fc.gain);
 #pragma unroll 4
   for (int k = n - 2; k >= 0; --k) {
-    y = (y - x[k * step]) * z;
+    const double c = next;
+    if (k > 0) next = x[(k - 1) * step];
+    y = (y - c) * z;
     put(k, y * fc.gain);
   }
 }
@@ -195,18 +200,21 @@ __global__ void filter_lines(const double* src, double* dst, int n, int64_t stri
     }
   } else {
     // the float coefficients are converted once per sample, over the doubles
-    // where those are not wanted themselves (conversions share the FP64 pipe)
+    // where those are not wanted themselves (conversions share the FP64 pipe); by
+    // memcpy, which keeps its order with the accesses of doubles to the same place
     const bool both = pd.out64 != nullptr;
     auto put = [&](int k, double v) {
+      const float f = (float)v;
       if (both) x[k * step] = v;
-      else *reinterpret_cast<float*>(x + k * step) = (float)v;
+      else memcpy(x + k * step, &f, sizeof(f));
     };
     if (n > 1) filter_line(x, n, step, fc, put);
     else put(0, x[0]);
     for_images(pd, axis, line, [&](int64_t o) {
       for (int k = 0; k < n; ++k) {
         const double v = both ? x[k * step] : 0.0;
-        const float f = both ? (float)v : *reinterpret_cast<const float*>(x + k * step);
+        float f = (float)v;
+        if (!both) memcpy(&f, x + k * step, sizeof(f));
         int64_t p[3];
         const int c = pad_images(k, n, p);
         for (int i = 0; i < c; ++i) store_padded(pd, o + p[i] * pd.ps[axis], v, f);
