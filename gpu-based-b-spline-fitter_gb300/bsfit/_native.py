@@ -36,6 +36,8 @@ SIGNATURES = {
     "bsfit_tune_rois_per_warp": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32]),
     "bsfit_tune_set": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int32,
                                       ctypes.c_int32]),
+    "bsfit_tune_restore": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int32,
+                                          ctypes.c_int32, ctypes.c_int64]),
     "bsfit_tune_get": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int64,
                                       ctypes.POINTER(ctypes.c_int32),
                                       ctypes.POINTER(ctypes.c_int32)]),

@@ -11,11 +11,16 @@ JSON cache file; ``apply_cache`` (or ``Model(..., tune_cache=path)``) puts the
 cached choices of this device back in force in a later process. Every
 configuration gives bit-identical results.
 
+A choice holds for the calls of the form that its sample had by default: one
+block per ROI (few ROIs), one warp per ROI, or several ROIs per warp (many). A
+file holds the last choice of a size, with the sample's number of ROIs; entries
+without one come from versions that had only the second form and hold for it.
+
 Cache file format (one file may hold several devices):
 
     {"format": "bsfit-tune-1",
      "devices": {"<device name>": {"<fit type>:<ROI size>":
-                  {"variant": v, "warps_per_block": w, "min_blocks": b, "ms": t}}}}
+                  {"variant": v, "warps_per_block": w, "min_blocks": b, "ms": t, "rois": n}}}}
 """
 import ctypes
 import json
@@ -57,8 +62,10 @@ def save_cache(path, cache):
 
 
 def record(cache, device, fittype, roi_size, choice):
-    cache.setdefault("devices", {}).setdefault(device, {})[cache_key(fittype, roi_size)] = {
-        k: choice[k] for k in ("variant", "warps_per_block", "min_blocks", "ms")}
+    entry = {k: choice[k] for k in ("variant", "warps_per_block", "min_blocks", "ms")}
+    if "rois" in choice:
+        entry["rois"] = int(choice["rois"])
+    cache.setdefault("devices", {}).setdefault(device, {})[cache_key(fittype, roi_size)] = entry
     return cache
 
 
@@ -71,18 +78,28 @@ def _set(fittype, roi_size, variant, wpb):
           "bsfit_tune_set")
 
 
+def _restore(fittype, roi_size, variant, wpb, rois):
+    check(_native.lib().bsfit_tune_restore(int(fittype), int(roi_size), int(variant), int(wpb), int(rois)),
+          "bsfit_tune_restore")
+
+
 def apply_cache(cache, device, setter=_set):
-    """Puts the cached choices for ``device`` in force (``setter(fittype,
-    roi_size, variant, warps_per_block)``, by default the library's
-    bsfit_tune_set on the current device); other devices' entries are ignored.
-    ``cache`` is a path or a loaded cache. Returns the number applied."""
+    """Puts the cached choices for ``device`` in force on the current device, each
+    for the form of the calls that it was measured in (or hands them to
+    ``setter(fittype, roi_size, variant, warps_per_block)``); other devices'
+    entries are ignored. ``cache`` is a path or a loaded cache. Returns the
+    number applied."""
     if isinstance(cache, (str, os.PathLike)):
         cache = load_cache(cache)
     n = 0
     for key, ch in cache.get("devices", {}).get(device, {}).items():
         try:
             ft, s = (int(x) for x in key.split(":"))
-            setter(ft, s, int(ch["variant"]), int(ch["warps_per_block"]))
+            v, w = int(ch["variant"]), int(ch["warps_per_block"])
+            if setter is _set:
+                _restore(ft, s, v, w, ch.get("rois", 0))
+            else:
+                setter(ft, s, v, w)
         except (ValueError, KeyError, TypeError):
             continue
         n += 1
@@ -119,9 +136,10 @@ def device_name():
 
 def autotune(model, rois, iterations, reps=3, cache=None, stream=None):
     """Times every configuration of ``model``'s fit type at the ROI size of
-    ``rois`` (a CUDA float32 tensor (N, s, s), a sample of the workload), puts
-    the fastest in force and returns it:
-    {"variant", "warps_per_block", "min_blocks", "ms", "candidates"} with
+    ``rois`` (a CUDA float32 tensor (N, s, s), a sample of the workload with about
+    the number of ROIs of the calls to come), puts the fastest in force for calls of
+    that form and returns it:
+    {"variant", "warps_per_block", "min_blocks", "ms", "rois", "candidates"} with
     candidates["v<variant>w<warps>"] the mean ms per call (None where the
     configuration cannot launch). With ``cache`` (a path) the choice is recorded
     there under this device's name."""
@@ -143,7 +161,7 @@ def autotune(model, rois, iterations, reps=3, cache=None, stream=None):
     choice = {"variant": bv.value, "warps_per_block": bw.value,
               "min_blocks": min_blocks(model.fittype, bv.value),
               "rois_per_warp": rois_per_warp(model.fittype, bv.value), "ms": bms.value,
-              "candidates": cand}
+              "rois": n, "candidates": cand}
     if cache is not None:
         c = load_cache(cache)
         record(c, device_name(), model.fittype, s, choice)

@@ -1264,10 +1264,24 @@ int bsfit_tune_set(int32_t fittype, int64_t roi_size, int32_t variant, int32_t w
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return BSFIT_E_NO_DEVICE;
   if (variant < 0) {
-    bsfit::tune_clear(fittype, (int)roi_size, dev);
+    bsfit::tune_clear(fittype, (int)roi_size, dev, bsfit::kAnyForm);
     return BSFIT_OK;
   }
-  if (!bsfit::tune_store(fittype, (int)roi_size, dev, bsfit::TuneConfig{variant, warps_per_block}))
+  if (!bsfit::tune_store(fittype, (int)roi_size, dev,
+                         bsfit::TuneConfig{variant, warps_per_block, bsfit::kAnyForm}))
+    return BSFIT_E_INVALID;
+  return BSFIT_OK;
+}
+
+int bsfit_tune_restore(int32_t fittype, int64_t roi_size, int32_t variant, int32_t warps_per_block,
+                       int64_t nfits) {
+  if (num_params(fittype) == 0) return BSFIT_E_UNSUPPORTED_FITTYPE;
+  if (roi_size < 1 || roi_size > kMaxRoi) return BSFIT_E_SUBREGION_SIZE;
+  if (nfits < 0) return BSFIT_E_INVALID;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return BSFIT_E_NO_DEVICE;
+  const bsfit::FitForm form = nfits > 0 ? bsfit::fit_form(fittype, (int)roi_size, nfits) : bsfit::kWarpForm;
+  if (!bsfit::tune_store(fittype, (int)roi_size, dev, bsfit::TuneConfig{variant, warps_per_block, form}))
     return BSFIT_E_INVALID;
   return BSFIT_OK;
 }
@@ -1276,8 +1290,8 @@ int bsfit_tune_get(int32_t fittype, int64_t roi_size, int32_t* variant, int32_t*
   if (!variant || !warps_per_block) return BSFIT_E_INVALID;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return BSFIT_E_NO_DEVICE;
-  bsfit::TuneConfig c{0, 0};
-  const bool found = bsfit::tune_lookup(fittype, (int)roi_size, dev, &c);
+  bsfit::TuneConfig c{};
+  const bool found = bsfit::tune_lookup(fittype, (int)roi_size, dev, bsfit::kAnyForm, &c);
   *variant = found ? c.variant : -1;
   *warps_per_block = found ? c.wpb : 0;
   return BSFIT_OK;
@@ -1305,11 +1319,13 @@ int bsfit_autotune_device(bsfit_model model, const float* d_rois, int64_t roi_si
   const int nv = bsfit::tune_num_variants(ft);
   const int wpbs[3] = {4, 2, 1};
   double best = -1.0;
-  bsfit::TuneConfig bc{0, 0};
+  // stored, while it is timed and after, for the form that such a call has by default
+  const bsfit::FitForm form = bsfit::fit_form(ft, (int)roi_size, nfits);
+  bsfit::TuneConfig bc{0, 0, form};
   int rc = BSFIT_OK;
   for (int v = 0; v < nv && rc == BSFIT_OK; ++v)
     for (int w = 0; w < 3 && rc == BSFIT_OK; ++w) {
-      bsfit::tune_store(ft, (int)roi_size, dev, bsfit::TuneConfig{v, wpbs[w]});
+      bsfit::tune_store(ft, (int)roi_size, dev, bsfit::TuneConfig{v, wpbs[w], form});
       double ms = -1.0;  // infeasible (shared memory or occupancy)
       int r = bsfit_fit_device(model, d_rois, roi_size, nfits, iterations, d_P, d_CRLB, d_LL, st);
       if (r == BSFIT_OK) {
@@ -1328,13 +1344,13 @@ int bsfit_autotune_device(bsfit_model model, const float* d_rois, int64_t roi_si
       if (all_ms) all_ms[v * 3 + w] = ms;
       if (ms > 0.0 && (best < 0.0 || ms < best)) {
         best = ms;
-        bc = bsfit::TuneConfig{v, wpbs[w]};
+        bc = bsfit::TuneConfig{v, wpbs[w], form};
       }
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc != BSFIT_OK || best < 0.0) {
-    bsfit::tune_clear(ft, (int)roi_size, dev);
+    bsfit::tune_clear(ft, (int)roi_size, dev, form);
     return rc != BSFIT_OK ? rc : BSFIT_E_CUDA;
   }
   bsfit::tune_store(ft, (int)roi_size, dev, bc);

@@ -195,29 +195,41 @@ WorkCounter::~WorkCounter() {
 cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t stream) {
   if (a.nseg <= 0) return cudaSuccess;
   const bool cap = a.warp_rois > 0;
-  // the autotuner's configuration for the largest ROI size of the batch (the
-  // capped form keeps the default kernel and takes the tuner's warps per block)
-  TuneConfig tc{0, 0};
-  int dev = 0;
-  if (!multi && cudaGetDevice(&dev) == cudaSuccess) tune_lookup(mode, a.s_max, dev, &tc);
-  if (cap) tc.variant = 0;
-  BatchKern kern = tc.variant > 0 ? batch_variant(mode, tc.variant) : batch_kern_default(mode, multi, cap);
+  BatchKern kern = batch_kern_default(mode, multi, cap);
   if (!kern) return cudaErrorInvalidValue;
-  const int rpw = tune_rois_per_warp(mode, tc.variant);
-  const int per_warp = tune_warp_floats(mode, tc.variant, a.s_max, false) * 4;
-  int wpb = 4, blocks_per_sm = 0, sms = 0;
-  cudaError_t e = pick_launch_wpb((const void*)kern, per_warp, multi ? 0 : tc.wpb, &wpb,
-                                  &blocks_per_sm, &sms);
-  if (e != cudaSuccess) return e;
-  const int smem = per_warp * wpb;
   int64_t total = 0;
   for (int i = 0; i < a.nseg; ++i) total += a.seg[i].n;
-  int64_t grid = (int64_t)sms * blocks_per_sm;
-  if (tc.variant <= 0 && !cap) {
-    bool taken = false;
-    e = launch_slots_batch(a, mode, multi, multi ? 0 : tc.wpb, total, grid * wpb, &taken, stream);
-    if (taken || e != cudaSuccess) return e;
+  int per_warp = warp_smem_floats(mode, a.s_max) * 4, rpw = 1;
+  int wpb = 4, bps = 0, sms = 0;
+  SlotLaunch slots{};
+  auto shape = [&](int want) {  // of one ROI per warp, and of the slots that could take its place
+    cudaError_t e = pick_launch_wpb((const void*)kern, per_warp, want, &wpb, &bps, &sms);
+    if (e == cudaSuccess && !cap)
+      e = pick_slots_batch(mode, a.s_max, multi, total, want, (int64_t)sms * bps * wpb, &slots);
+    return e;
+  };
+  cudaError_t e = shape(0);
+  if (e != cudaSuccess) return e;
+  // the autotuner's configuration for the largest ROI size of the batch (the
+  // capped form keeps the default kernel and takes the tuner's warps per block)
+  TuneConfig tc{};
+  int dev = 0;
+  if (!multi && cudaGetDevice(&dev) == cudaSuccess)
+    tune_lookup(mode, a.s_max, dev, slots.slots ? kSlotForm : kWarpForm, &tc);
+  if (cap) tc.variant = 0;
+  if (tc.variant > 0) {
+    kern = batch_variant(mode, tc.variant);
+    if (!kern) return cudaErrorInvalidValue;
+    rpw = tune_rois_per_warp(mode, tc.variant);
+    per_warp = tune_warp_floats(mode, tc.variant, a.s_max, false) * 4;
+    slots = SlotLaunch{};
+    e = pick_launch_wpb((const void*)kern, per_warp, tc.wpb, &wpb, &bps, &sms);
+  } else if (tc.wpb > 0) {
+    e = shape(tc.wpb);
   }
+  if (e != cudaSuccess) return e;
+  if (slots.slots) return launch_slots_batch(a, mode, multi, slots, stream);
+  int64_t grid = (int64_t)sms * bps;
   const int64_t need = (total + rpw * wpb - 1) / (rpw * wpb);
   if (need < grid) grid = need;
   // capped: enough blocks that every ROI is fitted
@@ -227,7 +239,7 @@ cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t 
     if (grid > 0x7fffffff) return cudaErrorInvalidValue;
   }
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, 32 * wpb, smem, stream>>>(a);
+  kern<<<(unsigned)grid, 32 * wpb, per_warp * wpb, stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -388,6 +400,31 @@ cudaError_t measure_fp32_peak(double* tflops) {
 
 // ---------------------------------------------------------------------------
 
+namespace {
+// One ROI per warp; null for what is not fitted (several starts with sCMOS variances).
+FitKern fit_kern_default(int mode, bool multi, bool var) {
+  if (var && multi) return nullptr;
+  if (mode == 6) return var ? fit_kernel<6, false, true> : fit_kernel<6, false>;
+  if (mode == 7) return var ? fit_kernel<7, false, true> : multi ? fit_kernel<7, true> : fit_kernel<7, false>;
+  if (mode == 8) return var ? fit_kernel<8, false, true> : multi ? fit_kernel<8, true> : fit_kernel<8, false>;
+  if (mode == kFit4Pi && !var) return multi ? fit_kernel<kFit4Pi, true> : fit_kernel<kFit4Pi, false>;
+  return nullptr;
+}
+}  // namespace
+
+FitForm fit_form(int mode, int s, int64_t nfits) {
+  TeamLaunch team{};
+  if (pick_team(mode, s, false, false, nfits, &team) == cudaSuccess && team.kern) return kTeamForm;
+  const FitKern kern = fit_kern_default(mode, false, false);
+  int wpb = 0, bps = 0, sms = 0;
+  SlotLaunch slots{};
+  if (kern &&
+      pick_launch((const void*)kern, warp_smem_floats(mode, s) * 4, &wpb, &bps, &sms) == cudaSuccess &&
+      pick_slots(mode, s, false, false, nfits, 0, (int64_t)sms * bps * wpb, &slots) == cudaSuccess && slots.slots)
+    return kSlotForm;
+  return kWarpForm;
+}
+
 cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream) {
   if (a.nfits <= 0) return cudaSuccess;
   if (a.flags & FLAG_PARITY) {
@@ -395,48 +432,62 @@ cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream) {
     if (a.var || a.n_starts > 1 || a.trace || a.m.fittype == kFit4Pi) return cudaErrorInvalidValue;
     return launch_fitdd(a, stream);
   }
-  {
-    bool taken = false;
-    const cudaError_t et = launch_team(a, &taken, stream);
-    if (taken || et != cudaSuccess) return et;
-  }
   const int mode = a.m.fittype;
-  const bool var = a.var != nullptr;
-  void (*kern)(FitArgs) = nullptr;
-  const bool multi = a.n_starts > 1;
-  if (var && multi) return cudaErrorInvalidValue;  // not combined
-  if (mode == 6) kern = var ? fit_kernel<6, false, true> : fit_kernel<6, false>;
-  else if (mode == 7) kern = var ? fit_kernel<7, false, true> : multi ? fit_kernel<7, true> : fit_kernel<7, false>;
-  else if (mode == 8) kern = var ? fit_kernel<8, false, true> : multi ? fit_kernel<8, true> : fit_kernel<8, false>;
-  else if (mode == kFit4Pi && !var) kern = multi ? fit_kernel<kFit4Pi, true> : fit_kernel<kFit4Pi, false>;
-  else return cudaErrorInvalidValue;
-  // The autotuner's configuration (kernel variant, warps per block) for this
-  // fit type and ROI size on this device, where one was chosen; otherwise the
-  // warps per block among 4, 2, 1 that keep the most warps resident per SM
-  // (shared memory per warp grows with s and the model).
-  TuneConfig tc{0, 0};
-  int dev = 0;
+  const bool var = a.var != nullptr, multi = a.n_starts > 1;
+  const bool plain = !a.trace && !a.flags;  // the forms besides one warp per ROI make no records
+  // The autotuner's configuration (kernel variant, warps per block) for this fit type
+  // and ROI size on this device, where one was chosen for the form that the call has by
+  // default.
   const bool tunable = !var && !multi && mode != kFit4Pi;
-  if (tunable && cudaGetDevice(&dev) == cudaSuccess && tune_lookup(mode, a.s, dev, &tc) &&
-      tc.variant > 0)
-    kern = fit_variant(mode, tc.variant);
-  if (!kern) return cudaErrorInvalidValue;
-  // ROIs per warp: 2 for the pair and packed variants of fit type 6
-  const int rpw = tunable ? tune_rois_per_warp(mode, tc.variant) : 1;
-  const int per_warp =
-      (tunable ? tune_warp_floats(mode, tc.variant, a.s, var) : warp_smem_floats(mode, a.s, var)) * 4;
-  int wpb = 4, blocks_per_sm = 0, sms = 0;
-  cudaError_t e = pick_launch_wpb((const void*)kern, per_warp, tunable ? tc.wpb : 0, &wpb,
-                                  &blocks_per_sm, &sms);
+  TuneConfig tc{};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const int smem = per_warp * wpb;
-  int64_t need = (a.nfits + rpw * wpb - 1) / (rpw * wpb);
-  int64_t grid = (int64_t)sms * blocks_per_sm;
-  if (tc.variant <= 0 && !a.trace && !a.flags) {
+  TeamLaunch team{};
+  if (plain) e = pick_team(mode, a.s, var, multi, a.nfits, &team);
+  if (e != cudaSuccess) return e;
+  if (team.kern) {
+    const bool tuned = tunable && tune_lookup(mode, a.s, dev, kTeamForm, &tc);
+    if (!tuned || (tc.form != kAnyForm && tc.variant == 0)) {
+      team.kern<<<(unsigned)a.nfits, team.threads, team.smem, stream>>>(a);
+      return cudaGetLastError();
+    }
+  }
+  FitKern kern = fit_kern_default(mode, multi, var);
+  if (!kern) return cudaErrorInvalidValue;
+  // The warps per block among 4, 2, 1 that keep the most warps resident per SM (shared
+  // memory per warp grows with s and the model), and the slots that could take the place
+  // of one ROI per warp.
+  int per_warp = warp_smem_floats(mode, a.s, var) * 4, rpw = 1;
+  int wpb = 4, bps = 0, sms = 0;
+  SlotLaunch slots{};
+  auto shape = [&](int want) {
+    cudaError_t r = pick_launch_wpb((const void*)kern, per_warp, want, &wpb, &bps, &sms);
+    if (r == cudaSuccess && plain && !team.kern)
+      r = pick_slots(mode, a.s, var, multi, a.nfits, want, (int64_t)sms * bps * wpb, &slots);
+    return r;
+  };
+  e = shape(0);
+  if (e != cudaSuccess) return e;
+  if (tunable && !team.kern) tune_lookup(mode, a.s, dev, slots.slots ? kSlotForm : kWarpForm, &tc);
+  if (tc.variant > 0) {
+    kern = fit_variant(mode, tc.variant);
+    if (!kern) return cudaErrorInvalidValue;
+    rpw = tune_rois_per_warp(mode, tc.variant);  // 2 for the pair and packed variants of fit type 6
+    per_warp = tune_warp_floats(mode, tc.variant, a.s, var) * 4;
+    slots = SlotLaunch{};
+    e = pick_launch_wpb((const void*)kern, per_warp, tc.wpb, &wpb, &bps, &sms);
+  } else if (tc.wpb > 0) {
+    e = shape(tc.wpb);
+  }
+  if (e != cudaSuccess) return e;
+  if (slots.slots) {
     bool taken = false;
-    e = launch_slots(a, tunable ? tc.wpb : 0, grid * wpb, &taken, stream);
+    e = launch_slots(a, slots, &taken, stream);
     if (taken || e != cudaSuccess) return e;
   }
+  const int64_t need = (a.nfits + rpw * wpb - 1) / (rpw * wpb);
+  int64_t grid = (int64_t)sms * bps;
   if (need < grid) grid = need;
   // More ROIs than resident warps: claim them dynamically (iteration counts
   // vary per ROI, and a fixed share per warp leaves the launch waiting on its
@@ -444,7 +495,7 @@ cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream) {
   FitArgs b = a;
   WorkCounter claim;
   if (need > grid) b.claim = claim.get(stream);
-  kern<<<(unsigned)grid, 32 * wpb, smem, stream>>>(b);
+  kern<<<(unsigned)grid, 32 * wpb, per_warp * wpb, stream>>>(b);
   return cudaGetLastError();
 }
 

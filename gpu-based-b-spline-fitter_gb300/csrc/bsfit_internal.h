@@ -190,9 +190,15 @@ int fit64_smem_bytes(int mode);
 int warp_smem_floats(int mode, int s, bool var = false, int stg = 0);
 cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t stream);
 cudaError_t launch_fit(const FitArgs& a, cudaStream_t stream);
-// The fit with one block per ROI, where that is the faster form (few ROIs);
-// otherwise *taken stays false and nothing is launched.
-cudaError_t launch_team(const FitArgs& a, bool* taken, cudaStream_t stream);
+using FitKern = void (*)(FitArgs);
+using BatchKern = void (*)(const BatchArgs);
+// The fit with one block per ROI (bsfit_team.cu): the kernel and block shape of a call,
+// kern null where that is not the faster form.
+struct TeamLaunch {
+  FitKern kern;
+  int threads, smem;
+};
+cudaError_t pick_team(int mode, int s, bool var, bool multi, int64_t nfits, TeamLaunch* t);
 // Double-float parity-grade fit of fit types 6, 7, 8 (plain ROIs, one start).
 cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream);
 int fitdd_smem_floats(int mode, int s);
@@ -212,13 +218,20 @@ class WorkCounter {
   unsigned long long* p_ = nullptr;
   cudaStream_t stream_ = nullptr;
 };
-// The fit with several ROIs in flight per warp (fit types 6, 7, 8), where that is
-// the faster form: `warps` is the number that the one-ROI-per-warp form keeps
-// resident, wpb the warps per block (0 to choose). Otherwise *taken stays false and
-// nothing is launched.
-cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, cudaStream_t stream);
-cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, int wpb, int64_t total, int64_t warps,
-                               bool* taken, cudaStream_t stream);
+// The fit with several ROIs in flight per warp (fit types 6, 7, 8; bsfit_slots.cu): the
+// slots per warp and launch shape, slots 0 where that is not the faster form. `warps` is
+// the number that the one-ROI-per-warp form keeps resident, wpb the warps per block (0 to
+// choose).
+struct SlotLaunch {
+  int slots, per_warp, wpb, bps, sms;
+};
+cudaError_t pick_slots(int mode, int s, bool var, bool multi, int64_t nfits, int wpb, int64_t warps,
+                       SlotLaunch* q);
+cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int64_t total, int wpb, int64_t warps,
+                             SlotLaunch* q);
+// *taken stays false when the pool has no work counter.
+cudaError_t launch_slots(const FitArgs& a, const SlotLaunch& q, bool* taken, cudaStream_t stream);
+cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, const SlotLaunch& q, cudaStream_t stream);
 // Launch shape of a fitter kernel (warps per block among 4, 2, 1 keeping the
 // most warps resident; blocks per SM; SM count), cached per kernel, size and
 // device.
@@ -227,15 +240,19 @@ cudaError_t pick_launch(const void* kern, int per_warp, int* wpb, int* bps, int*
 cudaError_t pick_launch_wpb(const void* kern, int per_warp, int force_wpb, int* wpb, int* bps,
                             int* sms);
 
+// The forms of a plain fit, by its number of ROIs: one block per ROI, one warp per ROI,
+// several ROIs per warp; kAnyForm: whatever the number.
+enum FitForm { kAnyForm = -1, kTeamForm, kWarpForm, kSlotForm };
+FitForm fit_form(int mode, int s, int64_t nfits);
+
 // Autotuner (bsfit_tune.cu): the launch configuration of the single-start FP32
-// fit kernels (plain and batched) per fit type, ROI size and device. variant 0
-// is the default kernel; wpb 0 lets the occupancy choice stand.
+// fit kernels (plain and batched) per fit type, ROI size, device and form. variant 0
+// is the form's default kernel; wpb 0 lets the occupancy choice stand.
 struct TuneConfig {
   int variant;
   int wpb;
+  FitForm form;  // kAnyForm: the caller's own choice, for every call of the size
 };
-using FitKern = void (*)(FitArgs);
-using BatchKern = void (*)(const BatchArgs);
 int tune_num_variants(int mode);
 int tune_min_blocks(int mode, int variant);
 // 1 when the variant stages the 5D gathers through shared memory (its
@@ -248,9 +265,12 @@ int tune_warp_floats(int mode, int variant, int s, bool var);
 FitKern fit_variant(int mode, int variant);     // variant >= 1
 BatchKern batch_variant(int mode, int variant);  // variant >= 1
 BatchKern batch_kern_default(int mode, bool multi, bool cap);
-bool tune_lookup(int mode, int s, int dev, TuneConfig* out);
+// The configuration of a call whose default form is `form`: the caller's choice, else
+// the one tuned in that form. With kAnyForm: the caller's, else the last one stored.
+bool tune_lookup(int mode, int s, int dev, FitForm form, TuneConfig* out);
+// Stores c for its form; kAnyForm takes the place of all, and gives way to any other.
 bool tune_store(int mode, int s, int dev, TuneConfig c);
-void tune_clear(int mode, int s, int dev);
+void tune_clear(int mode, int s, int dev, FitForm form);  // kAnyForm: all forms
 cudaError_t measure_fp32_peak(double* tflops);
 // FP32 FMA throughput of scalar and of paired (FFMA2) FMA chains, TFLOP/s.
 cudaError_t measure_fp32_peak2(double* scalar, double* paired);

@@ -18,9 +18,12 @@ FitKern slot_kern_of(bool multi, bool var) {
   return slot_kernel<MODE, false, false, B>;
 }
 
-struct SlotLaunch {
-  int slots, per_warp, wpb, bps, sms;
-};
+FitKern slot_kern(int mode, bool multi, bool var) {
+  return mode == 6   ? slot_kern_of<6>(false, var)
+         : mode == 7 ? slot_kern_of<7>(multi, var)
+         : mode == 8 ? slot_kern_of<8>(multi, var)
+                     : nullptr;
+}
 
 // The slot form's place. Measured on GB300 (ms; one ROI per warp / slot form,
 // W the warps that the first keeps resident):
@@ -53,7 +56,7 @@ constexpr int64_t kSparePerWarp = 2;
 // (to 5%), or, where the slots' shared memory leaves none, the most that keep 85% of
 // them (21 px 3D ROIs: 17 warps per SM against 20, and still 1.5% faster). q->slots
 // 0: not even two do. more: floats per warp besides the layout's.
-cudaError_t pick_slots(const void* kern, int mode, int s, bool var, bool multi, int more, int wpb,
+cudaError_t most_slots(const void* kern, int mode, int s, bool var, bool multi, int more, int wpb,
                        int64_t warps, SlotLaunch* q) {
   for (int percent : {95, 85})
     for (int r = kMaxSlots; r >= 2; --r) {
@@ -68,46 +71,42 @@ cudaError_t pick_slots(const void* kern, int mode, int s, bool var, bool multi, 
 
 }  // namespace
 
-cudaError_t launch_slots(const FitArgs& a, int wpb, int64_t warps, bool* taken, cudaStream_t stream) {
-  *taken = false;
-  const bool var = a.var != nullptr, multi = a.n_starts > 1;
-  const int mode = a.m.fittype;
-  if (a.nfits < kEnough * warps) return cudaSuccess;
-  const FitKern kern = mode == 6   ? slot_kern_of<6>(false, var)
-                       : mode == 7 ? slot_kern_of<7>(multi, var)
-                       : mode == 8 ? slot_kern_of<8>(multi, var)
-                                   : nullptr;
-  if (!kern) return cudaSuccess;
-  SlotLaunch q{};
-  const cudaError_t e = pick_slots((const void*)kern, mode, a.s, var, multi, 0, wpb, warps, &q);
-  if (e != cudaSuccess || q.slots < 2) return e;
+cudaError_t pick_slots(int mode, int s, bool var, bool multi, int64_t nfits, int wpb, int64_t warps,
+                       SlotLaunch* q) {
+  *q = SlotLaunch{};
+  if (nfits < kEnough * warps) return cudaSuccess;
+  const FitKern kern = slot_kern(mode, multi, var);
+  return kern ? most_slots((const void*)kern, mode, s, var, multi, 0, wpb, warps, q) : cudaSuccess;
+}
+
+cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int64_t total, int wpb, int64_t warps,
+                             SlotLaunch* q) {
+  *q = SlotLaunch{};
+  if (total < (mode == 6 ? kEnoughBatch3D : kEnough) * warps) return cudaSuccess;
+  const BatchKern kern = slot_batch_kern(mode, multi);
+  return kern ? most_slots((const void*)kern, mode, s_max, false, multi, kSegWords, wpb, warps, q) : cudaSuccess;
+}
+
+cudaError_t launch_slots(const FitArgs& a, const SlotLaunch& q, bool* taken, cudaStream_t stream) {
   FitArgs b = a;
   WorkCounter claim;
   b.slots = q.slots;
   b.claim = claim.get(stream);
-  if (!b.claim) return cudaSuccess;
+  *taken = b.claim != nullptr;
+  if (!*taken) return cudaSuccess;
   const int64_t grid = (int64_t)q.sms * q.bps;
   b.spare = kSparePerWarp * grid * q.wpb;
-  *taken = true;
-  kern<<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
+  slot_kern(a.m.fittype, a.n_starts > 1, a.var != nullptr)
+      <<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
   return cudaGetLastError();
 }
 
-cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, int wpb, int64_t total, int64_t warps,
-                               bool* taken, cudaStream_t stream) {
-  *taken = false;
-  if (total < (mode == 6 ? kEnoughBatch3D : kEnough) * warps) return cudaSuccess;
-  const BatchKern kern = slot_batch_kern(mode, multi);
-  if (!kern) return cudaSuccess;
-  SlotLaunch q{};
-  const cudaError_t e = pick_slots((const void*)kern, mode, a.s_max, false, multi, kSegWords, wpb, warps, &q);
-  if (e != cudaSuccess || q.slots < 2) return e;
+cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, const SlotLaunch& q, cudaStream_t stream) {
   BatchArgs b = a;
   b.slots = q.slots;
   const int64_t grid = (int64_t)q.sms * q.bps;
   b.spare = kSparePerWarp * grid * q.wpb;
-  *taken = true;
-  kern<<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
+  slot_batch_kern(mode, multi)<<<(unsigned)grid, 32 * q.wpb, q.per_warp * q.wpb, stream>>>(b);
   return cudaGetLastError();
 }
 

@@ -63,29 +63,23 @@ constexpr Form kForms[] = {
 
 }  // namespace
 
-cudaError_t launch_team(const FitArgs& a, bool* taken, cudaStream_t stream) {
-  *taken = false;
-  const bool var = a.var != nullptr, multi = a.n_starts > 1;
-  const int mode = a.m.fittype;
-  if (a.trace || a.flags || (var && multi) || (var && mode == kFit4Pi) || (multi && mode == 6))
-    return cudaSuccess;
+cudaError_t pick_team(int mode, int s, bool var, bool multi, int64_t nfits, TeamLaunch* t) {
+  *t = TeamLaunch{nullptr, 0, 0};
+  if ((var && multi) || (var && mode == kFit4Pi) || (multi && mode == 6)) return cudaSuccess;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   e = sm_count(dev, &sms);
   if (e != cudaSuccess) return e;
-  const double n = (double)a.nfits / sms;
+  const double n = (double)nfits / sms;
   if (n > 9.0) return cudaSuccess;  // past every form
-  // a configuration that was put in force for this size is kept
-  TuneConfig tc{0, 0};
-  if (tune_lookup(mode, a.s, dev, &tc)) return cudaSuccess;
   for (const Form& f : kForms) {
     if (f.mode != mode || n > f.most) continue;
     const int T = f.warps;
     TeamKern kern = T == 16 ? team_kern16(mode, multi, var) : T == 8 ? team_kern8(mode, multi, var)
                                                                      : team_kern4(mode, f.blocks, multi, var);
     if (!kern) kern = team_kern4_dense(mode, f.blocks, multi, var);
-    const int per_warp = ((make_team_layout(mode, a.s, var, T).total * 4 + T - 1) / T + 15) & ~15;
+    const int per_warp = ((make_team_layout(mode, s, var, T).total * 4 + T - 1) / T + 15) & ~15;
     if (!kern || per_warp * T > kTeamMaxShared) continue;
     int wpb = 0, bps = 0;
     e = pick_launch_wpb((const void*)kern, per_warp, T, &wpb, &bps, &sms);
@@ -94,9 +88,8 @@ cudaError_t launch_team(const FitArgs& a, bool* taken, cudaStream_t stream) {
     // three waves still win (one warp / team, us: 4Pi 24 px, 300 ROIs, one block per
     // SM, 1196 / 529, but 600 ROIs 1226 / 1259; 3D 33 px, 800 ROIs 542 / 331).
     if (n > 3.0 * bps) continue;
-    *taken = true;
-    kern<<<(unsigned)a.nfits, 32 * T, per_warp * T, stream>>>(a);
-    return cudaGetLastError();
+    *t = TeamLaunch{kern, 32 * T, per_warp * T};
+    return cudaSuccess;
   }
   return cudaSuccess;
 }

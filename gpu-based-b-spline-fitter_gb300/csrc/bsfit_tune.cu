@@ -17,11 +17,18 @@
 //    that does not grow with the ROI between two ROIs at twice the shared
 //    memory per warp, or both on all 32 lanes in the two halves of paired FP32
 //    operations (bsfit_pack.cuh), which shares the whole evaluation.
-// Variant 0 is the default: one ROI per warp (bsfit_fit.cu), or several in flight
-// per warp for calls of many ROIs (bsfit_slots.cu); this file instantiates the
-// others. Every variant runs the same code, so results are bit-identical
-// across configurations. A table per (fit type, ROI size, device) holds the
-// chosen configuration; launch_fit and launch_batch consult it.
+// Variant 0 is the default: one ROI per warp (bsfit_fit.cu), one per block for calls of
+// few ROIs (bsfit_team.cu), or several in flight per warp for calls of many
+// (bsfit_slots.cu); this file instantiates the others. Every variant runs the same
+// code, so results are bit-identical across configurations. A table per (fit type, ROI
+// size, device, form) holds the chosen configuration; launch_fit and launch_batch
+// consult it.
+//
+// A choice holds for the calls of the form that it was measured in. Held for every
+// count of the size, one tuned on 100,000 13 px 3D ROIs sent a call of one ROI from
+// 28 us back to 54, and 5D 17 px tuned on 5,000 ROIs (variant 1) sent 50,000 from 37.3 ms
+// to 39.1; the other way round, 10,000 5D ROIs of 21 px are faster with variant 1 than
+// in slots (11.2 ms against 12.6), which a tuner that saw such a call keeps.
 #include <mutex>
 
 #include "bsfit_fit_kernels.cuh"
@@ -47,6 +54,7 @@ constexpr bool kStaged8[4] = {false, false, true, true};
 struct Entry {
   int mode, s, dev;
   TuneConfig c;
+  bool is(int m, int size, int d) const { return mode == m && s == size && dev == d; }
 };
 std::mutex g_tune_mu;
 constexpr int kMaxEntries = 512;
@@ -114,37 +122,43 @@ BatchKern batch_variant(int mode, int variant) {
   }
 }
 
-bool tune_lookup(int mode, int s, int dev, TuneConfig* out) {
+bool tune_lookup(int mode, int s, int dev, FitForm form, TuneConfig* out) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  for (int i = 0; i < g_ntune; ++i)
-    if (g_tune[i].mode == mode && g_tune[i].s == s && g_tune[i].dev == dev) {
+  // kept in the order of their storing
+  for (int i = g_ntune - 1; i >= 0; --i)
+    if (g_tune[i].is(mode, s, dev) &&
+        (form == kAnyForm || g_tune[i].c.form == kAnyForm || g_tune[i].c.form == form)) {
       *out = g_tune[i].c;
       return true;
     }
   return false;
 }
 
+namespace {
+// Takes out the entries of a size: form's and the caller's, or all.
+void drop(int mode, int s, int dev, FitForm form) {
+  int n = 0;
+  for (int i = 0; i < g_ntune; ++i)
+    if (!g_tune[i].is(mode, s, dev) ||
+        !(form == kAnyForm || g_tune[i].c.form == kAnyForm || g_tune[i].c.form == form))
+      g_tune[n++] = g_tune[i];
+  g_ntune = n;
+}
+}  // namespace
+
 bool tune_store(int mode, int s, int dev, TuneConfig c) {
   if (c.variant < 0 || c.variant >= tune_num_variants(mode)) return false;
   if (c.wpb != 0 && c.wpb != 1 && c.wpb != 2 && c.wpb != 4) return false;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  for (int i = 0; i < g_ntune; ++i)
-    if (g_tune[i].mode == mode && g_tune[i].s == s && g_tune[i].dev == dev) {
-      g_tune[i].c = c;
-      return true;
-    }
+  drop(mode, s, dev, c.form);
   if (g_ntune >= kMaxEntries) return false;
   g_tune[g_ntune++] = Entry{mode, s, dev, c};
   return true;
 }
 
-void tune_clear(int mode, int s, int dev) {
+void tune_clear(int mode, int s, int dev, FitForm form) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  for (int i = 0; i < g_ntune; ++i)
-    if (g_tune[i].mode == mode && g_tune[i].s == s && g_tune[i].dev == dev) {
-      g_tune[i] = g_tune[--g_ntune];
-      return;
-    }
+  drop(mode, s, dev, form);
 }
 
 }  // namespace bsfit

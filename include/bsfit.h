@@ -370,7 +370,11 @@ int bsfit_batch_fit_device_static(const bsfit_segment* segs, int32_t nseg, void*
  * warp, one or two: bsfit_tune_rois_per_warp) and the warps per block (4, 2 or
  * 1; 0 keeps the occupancy choice). Variant 0 with 0 warps per block is the
  * default. Every configuration gives bit-identical results. The batched form
- * uses the configuration of its largest ROI size.
+ * uses the configuration of its largest ROI size. By default a call's form follows
+ * its number of ROIs: one block per ROI (few), one warp per ROI, several ROIs per
+ * warp (many). A configuration that was tuned holds for the calls of the form that
+ * its sample had; one that bsfit_tune_set sets holds for every number of ROIs, and
+ * has calls of few ROIs fitted with one warp per ROI.
  */
 int bsfit_tune_num_variants(int32_t fittype);                  /* 0 if none */
 int bsfit_tune_min_blocks(int32_t fittype, int32_t variant);   /* 0 if out of range */
@@ -378,12 +382,17 @@ int bsfit_tune_rois_per_warp(int32_t fittype, int32_t variant); /* 0 if out of r
 /* Sets the configuration for (fittype, roi_size) on the current device;
  * variant -1 restores the default. */
 int bsfit_tune_set(int32_t fittype, int64_t roi_size, int32_t variant, int32_t warps_per_block);
-/* The configuration in force: variant -1 when the default applies. */
+/* Sets it as bsfit_autotune_device with a sample of nfits ROIs would have (for the
+ * calls of that sample's form); nfits 0: for the calls with one warp per ROI. */
+int bsfit_tune_restore(int32_t fittype, int64_t roi_size, int32_t variant, int32_t warps_per_block,
+                       int64_t nfits);
+/* The configuration in force (the last one set, where several forms have one):
+ * variant -1 when the default applies. */
 int bsfit_tune_get(int32_t fittype, int64_t roi_size, int32_t* variant, int32_t* warps_per_block);
 /* Times every configuration on the caller's ROIs (a sample of the workload:
  * one untimed and `reps` timed bsfit_fit_device calls each, CUDA events on
- * `stream`), sets the fastest for (fit type, roi_size) on the current device
- * and returns it. all_ms (optional, 3 * bsfit_tune_num_variants doubles):
+ * `stream`), sets the fastest for (fit type, roi_size) on the current device, for
+ * calls of the form that such a sample has by default, and returns it. all_ms (optional, 3 * bsfit_tune_num_variants doubles):
  * mean ms per call of (variant v, warps per block 4 / 2 / 1) at
  * [v * 3 + {0, 1, 2}], -1 where the configuration cannot launch. The outputs
  * hold the last timed call's results. Synchronises the stream. */
