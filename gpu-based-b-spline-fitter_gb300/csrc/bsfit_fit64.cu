@@ -22,15 +22,15 @@
 // the double build it follows. The only other source of difference is the
 // last bit of log().
 //
-// Layout: one block of kTeam = 4 warps per ROI: the sums' dependent adds let one
-// warp use a quarter of the SM's FP64 rate, and a call of few ROIs, or the last ones
-// of a large call, lasts as long as one fit. Threads evaluate pixels
-// 128 at a time and publish each pixel's terms in a shared row (its deviance term,
+// Layout: one block of four warps per ROI (TEAM; two or one for some counts,
+// launch_mode): the sums' dependent adds let one warp use a quarter of the SM's FP64
+// rate, and a call of few ROIs, or the last ones of a large call, lasts as long as one
+// fit. Threads evaluate pixels 128 at a time and publish each pixel's terms in a shared row (its deviance term,
 // t1 * dudt[l], and (t2 * dudt[l]) * dudt[m], the products the reference adds); the
 // sums are owned one per thread and accumulated over the rows in pixel order, so
-// every sum has the reference's order. One warp, another from ROI to ROI so that the
-// four units share it, forms the sums and runs the LM control and the small dense
-// solves, lane l on parameter or row l, on shared state: an FP64 instruction costs
+// every sum has the reference's order. The lead warp, another from ROI to ROI so that the
+// four units share it, forms the sums (5D: 45, with the next one) and runs the LM control
+// and the small dense solves, lane l on parameter or row l, on shared state: an FP64 instruction costs
 // the same for one lane as for 32. Coefficients are a double copy of the model's table followed by
 // one table per axis of the neighbour differences (-c[i]) + c[i + stride] the
 // derivative terms use (computed once per model, the same double operation). ROIs are
@@ -80,8 +80,6 @@ constexpr float kPIf = 3.141592f;
 constexpr float kTOLf = 1e-6f;
 constexpr float kTOL1f = 1e-5f;
 
-constexpr int kTeam = 4, kThreads = 32 * kTeam;
-
 // LM state of one block, written by its lead warp (the owners of the sums write err / jac
 // / hes / M / div between two block barriers).
 struct LMState {
@@ -95,9 +93,10 @@ struct LMState {
 static_assert(sizeof(LMState) % 16 == 0, "LMState keeps the tables 16-byte aligned");
 constexpr int kLMDoubles = (int)(sizeof(LMState) / sizeof(double));
 
-template <int MODE>
+template <int MODE, int TEAM>
 struct F64Layout {
   using TR = F64Traits<MODE>;
+  static constexpr int kThreads = 32 * TEAM;
   static constexpr int D = TR::D, NV = TR::NV;
   static constexpr int B = 1 << D, BB = B * B;
   static constexpr int WT = (D + 1) * BB;             // wf, then wd[0..D-1]
@@ -175,10 +174,10 @@ __device__ __forceinline__ double axis_weight(double frac, int kind, int v) {
 // Tensor-product tables of D axes from ax[]: entry B*n + b, n the loop index
 // (axis a at v = bit a of n, plus 1), b the side bits; the products run over
 // the axes left to right.
-template <int D>
+template <int D, int THREADS>
 __device__ __forceinline__ void build_tables(const double* ax, double* W) {
   constexpr int B = 1 << D, BB = B * B;
-  for (int e = threadIdx.x; e < BB; e += kThreads) {
+  for (int e = threadIdx.x; e < BB; e += THREADS) {
     const int n = e >> D, b = e & (B - 1);
     double val[D], der[D];
 #pragma unroll
@@ -283,9 +282,10 @@ struct Fit64Ctx {
   int s;
 };
 
-template <int MODE>
+template <int MODE, int TEAM>
 struct Team64 {
-  using L = F64Layout<MODE>;
+  using L = F64Layout<MODE, TEAM>;
+  static constexpr int kThreads = L::kThreads;
   static constexpr int D = L::D, NV = L::NV, RW = L::RW;
   LMState& st;
   double* wt;
@@ -355,8 +355,8 @@ struct Team64 {
       st.frame[6] = (MODE == 8) ? th[7] : 0.0;
     }
     __syncthreads();
-    build_tables<D>(ax, wt);
-    if constexpr (MODE == 8) build_tables<3>(ax, wt3);
+    build_tables<D, kThreads>(ax, wt);
+    if constexpr (MODE == 8) build_tables<3, kThreads>(ax, wt3);
     __syncthreads();
   }
 
@@ -385,8 +385,8 @@ struct Team64 {
     }
   }
 
-  // The pixels of one plane, in the reference's order (ii outer, jj inner), 128
-  // at a time: each thread publishes its pixel's terms in a row (the deviance
+  // The pixels of one plane, in the reference's order (ii outer, jj inner), one per
+  // thread at a time: each thread publishes its pixel's terms in a row (the deviance
   // term, t1 * dudt[l] and (t2 * dudt[l]) * dudt[m]; or the log-likelihood term,
   // its use flag and (dudt[m] * dudt[l]) / model), then every owner adds its
   // entry of the rows in pixel order to acc.
@@ -816,16 +816,14 @@ __device__ void init_state(LMState& st) {
   }
 }
 
-// Resident blocks per SM that the registers are held to: four for 3D and 4D (128
-// registers, no spills; 4D at three blocks, 168 registers, needs a second wave from
-// 457 ROIs: 600 ROIs of 13 px, three iterations, 4.16 ms against 2.92).
-template <int MODE>
-__global__ void __launch_bounds__(kThreads, MODE == 6 || MODE == 7 ? 4 : MODE == 8 ? 2 : 3) fit64_kernel(const __grid_constant__ Fit64Args a) {
-  using L = F64Layout<MODE>;
+// BLOCKS: the resident blocks per SM that the registers are held to.
+template <int MODE, int TEAM, int BLOCKS>
+__global__ void __launch_bounds__(32 * TEAM, BLOCKS) fit64_kernel(const __grid_constant__ Fit64Args a) {
+  using L = F64Layout<MODE, TEAM>;
   constexpr int NV = L::NV;
   extern __shared__ double smem64[];
   const int lane = threadIdx.x & 31;
-  Team64<MODE> w(smem64);
+  Team64<MODE, TEAM> w(smem64);
   LMState& st = w.st;
   Fit64Ctx cx;
   cx.a = &a;
@@ -844,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 6 || MODE == 7 ? 4 : MODE ==
     cx.var = a.var ? a.var + roi * s2 : nullptr;
     cx.dT = (MODE == kFit4Pi) ? a.dT + roi * (int64_t)(k4PiChannels * NV) : nullptr;
     // the warp that does the LM steps and forms the sums, another from ROI to ROI
-    const int lead_warp = (int)(roi & (kTeam - 1));
+    const int lead_warp = (int)(roi & (TEAM - 1));
     const bool lead = (int)(threadIdx.x >> 5) == lead_warp;
     w.assign(lead_warp);
     if (lead) {
@@ -977,18 +975,20 @@ __global__ void widen_kernel(const float* __restrict__ src, double* __restrict__
   }
 }
 
-// Blocks per SM and SM count of fit64_kernel<MODE> on a device, computed once
-// (the kernel's shared-memory limit is set then), so later launches, including
-// ones captured into a CUDA graph, make no attribute or occupancy calls.
+// Blocks per SM and SM count of a kernel on a device, computed once (the kernel's
+// shared-memory limit is set then), so later launches, including ones captured into a
+// CUDA graph, make no attribute or occupancy calls.
 struct Launch64 {
   int dev = -1, per_sm = 0, sms = 0;
 };
 std::mutex g_launch64_mu;
 
-template <int MODE>
-cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
-  using L = F64Layout<MODE>;
-  const size_t smem = (size_t)L::total * sizeof(double);
+// Fits with TEAM warps per ROI. With `even`, only where the blocks hold all ROIs at
+// once; *taken stays false otherwise.
+template <int MODE, int TEAM, int BLOCKS>
+cudaError_t launch64(const Fit64Args& a, bool even, bool* taken, cudaStream_t stream) {
+  constexpr int threads = 32 * TEAM;
+  const size_t smem = (size_t)F64Layout<MODE, TEAM>::total * sizeof(double);
   static Launch64 cache[8];  // per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -999,11 +999,11 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
     std::lock_guard<std::mutex> lk(g_launch64_mu);
     Launch64& c = cache[dev];
     if (c.dev != dev) {
-      e = cudaFuncSetAttribute(fit64_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(fit64_kernel<MODE, TEAM, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem);
       if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev);
       if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.per_sm, fit64_kernel<MODE>, kThreads,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.per_sm, fit64_kernel<MODE, TEAM, BLOCKS>, threads,
                                                           smem);
       if (e != cudaSuccess) return e;
       c.dev = dev;
@@ -1013,6 +1013,7 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
   }
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int64_t cap = (int64_t)sms * per_sm;
+  if (even && a.nfits > cap) return cudaSuccess;
   const int64_t grid = a.nfits < cap ? a.nfits : cap;
   // More ROIs than resident blocks: claimed one at a time, but from fixed shares in a
   // capture, which then records the launch alone (a graph with the counter's memory
@@ -1023,18 +1024,59 @@ cudaError_t launch64(const Fit64Args& a, cudaStream_t stream) {
   if (a.nfits > grid && cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
       capture == cudaStreamCaptureStatusNone)
     b.claim = claim.get(stream);
-  fit64_kernel<MODE><<<(unsigned)grid, kThreads, smem, stream>>>(b);
+  *taken = true;
+  fit64_kernel<MODE, TEAM, BLOCKS><<<(unsigned)grid, threads, smem, stream>>>(b);
   return cudaGetLastError();
+}
+
+// Four warps per ROI are the fastest for one ROI and for many, where the claims even the
+// fits' lengths out. Fits of few iterations all make as many, so they run in waves: a
+// call of a little more than a wave takes two, and one whose ROIs two warps or one (4D,
+// 4Pi) hold at once is faster so. Measured (GB300, ms, the same number of iterations in
+// all fits; one warp per ROI held to 140 registers / four warps / two / one):
+//   4Pi 12 px  4 ROIs per SM, 6 iterations 17.5 / 26.7 / 16.7 / 17.3    10, 6: 42.0 / 53.3 / 48.0 / 41.3
+//   4D  13 px  5, 6: 6.82 / 7.96 / 6.15 / 6.73    9, 6: 11.6 / 12.3 / 11.8 / 11.3
+//   3D  17 px  5, 6: 4.42 / 3.80 / 2.70           7 px, 8, 1: 0.439 / 0.462 / 0.395
+//   5D  13 px  3, 6: 24.5 / 23.9 / 18.0
+// With more iterations than most fits need the four warps win by the longest fits; the
+// line lies about where they do (cap of iterations, four warps / two): 3D 11 px, 7.5 per
+// SM, 9 2.39 / 2.37, 13 2.61 / 2.70; 4D 13 px, 6 per SM, 45 47.7 / 43.0, 60 54.1 / 56.8;
+// 5D 13 px, 2.2 per SM, 30 77.6 / 70.9, 45 100 / 104; 4Pi 12 px, 4 per SM, 60 160 / 127,
+// 100 182 / 174, 3.3 per SM, 100 148 / 163.
+template <int MODE>
+cudaError_t launch_mode(const Fit64Args& a, cudaStream_t stream) {
+  const int steps = a.handoff && a.handoff_iters < a.iterations ? a.handoff_iters : a.iterations;
+  const bool alike = steps <= (MODE == 6 ? 10 : MODE == 7 ? 50 : MODE == 8 ? 30 : 80);
+  bool taken = false;
+  cudaError_t e = cudaSuccess;
+  if constexpr (MODE == 6) {
+    if (alike) e = launch64<6, 4, 4>(a, true, &taken, stream);
+    if (alike && !taken && e == cudaSuccess) e = launch64<6, 2, 8>(a, true, &taken, stream);
+    if (!taken && e == cudaSuccess) e = launch64<6, 4, 4>(a, false, &taken, stream);
+  } else if constexpr (MODE == 8) {
+    if (alike) e = launch64<8, 4, 2>(a, true, &taken, stream);
+    if (alike && !taken && e == cudaSuccess) e = launch64<8, 2, 4>(a, true, &taken, stream);
+    if (!taken && e == cudaSuccess) e = launch64<8, 4, 2>(a, false, &taken, stream);
+  } else {
+    // 4D at four blocks spills 96 bytes; three blocks (162 registers, no spills) need a
+    // second wave from 457 ROIs: 600 of 13 px, three iterations, 4.16 ms against 2.92
+    constexpr int B = MODE == 7 ? 4 : 3;
+    if (alike) e = launch64<MODE, 4, B>(a, true, &taken, stream);
+    if (alike && !taken && e == cudaSuccess) e = launch64<MODE, 2, 8>(a, true, &taken, stream);
+    if (alike && !taken && e == cudaSuccess) e = launch64<MODE, 1, 11>(a, true, &taken, stream);
+    if (!taken && e == cudaSuccess) e = launch64<MODE, 4, B>(a, false, &taken, stream);
+  }
+  return e;
 }
 
 }  // namespace
 
 int fit64_smem_bytes(int mode) {
   switch (mode) {
-    case 6: return F64Layout<6>::total * 8;
-    case 7: return F64Layout<7>::total * 8;
-    case 8: return F64Layout<8>::total * 8;
-    case kFit4Pi: return F64Layout<kFit4Pi>::total * 8;
+    case 6: return F64Layout<6, 4>::total * 8;
+    case 7: return F64Layout<7, 4>::total * 8;
+    case 8: return F64Layout<8, 4>::total * 8;
+    case kFit4Pi: return F64Layout<kFit4Pi, 4>::total * 8;
     default: return 0;
   }
 }
@@ -1054,10 +1096,10 @@ cudaError_t widen_to_f64(const float* src, double* dst, int64_t total, int naxes
 cudaError_t launch_fit64(const Fit64Args& a, cudaStream_t stream) {
   if (a.nfits <= 0) return cudaSuccess;
   switch (a.m.fittype) {
-    case 6: return launch64<6>(a, stream);
-    case 7: return launch64<7>(a, stream);
-    case 8: return launch64<8>(a, stream);
-    case kFit4Pi: return launch64<kFit4Pi>(a, stream);
+    case 6: return launch_mode<6>(a, stream);
+    case 7: return launch_mode<7>(a, stream);
+    case 8: return launch_mode<8>(a, stream);
+    case kFit4Pi: return launch_mode<kFit4Pi>(a, stream);
     default: return cudaErrorInvalidValue;
   }
 }
