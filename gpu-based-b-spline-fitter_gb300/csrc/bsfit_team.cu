@@ -19,7 +19,7 @@ TeamKern team_kern8(int mode, bool multi, bool var) {
 }
 
 // A form: warps per block, blocks per SM that it is compiled for, and the most ROIs
-// per SM that it is used for. The first that fits is taken. Measured (GB300, 152
+// per SM that it is used for. The first whose range holds the call is taken. Measured (GB300, 152
 // SMs; us per call, ROIs of 13 px for 3D and 4D, 17 px for 5D, 4 x 16 px for 4Pi;
 // warps/blocks):
 //
@@ -60,6 +60,7 @@ constexpr Form kForms[] = {
     {8, 16, 1, 1.0},      {8, 8, 2, 2.0},       {8, 4, 3, 3.0}, {8, 4, 4, 4.0}, {8, 4, 5, 5.0},
     {kFit4Pi, 16, 1, 1.0}, {kFit4Pi, 8, 2, 2.0}, {kFit4Pi, 4, 4, 9.0},
 };
+constexpr double kMostWaves = 7.0;
 
 }  // namespace
 
@@ -73,8 +74,19 @@ cudaError_t pick_team(int mode, int s, bool var, bool multi, int64_t nfits, Team
   if (e != cudaSuccess) return e;
   const double n = (double)nfits / sms;
   if (n > 9.0) return cudaSuccess;  // past every form
-  for (const Form& f : kForms) {
-    if (f.mode != mode || n > f.most) continue;
+  constexpr int kNumForms = (int)(sizeof(kForms) / sizeof(kForms[0]));
+  int at = 0;
+  while (at < kNumForms && (kForms[at].mode != mode || n > kForms[at].most)) ++at;
+  if (at == kNumForms) return cudaSuccess;
+  // Large ROIs: fewer blocks than a form is compiled for fit an SM's shared memory, and
+  // unless they still hold the call in one wave, its registers are short for nothing:
+  // the next sparser form takes its place, down to the first. Measured (us; one warp /
+  // the form by count / this): 5D 27 px, 760 ROIs 2,440 / 3,400 / 2,300, 33 px, 684
+  // 3,900 / 5,150 / 2,885; 4Pi 24 px, 530 5,200 / 5,200 / 3,100; 3D 51 px, 760 1,280 /
+  // 1,290 / 733.
+  int blocks = 0;
+  for (; at >= 0 && kForms[at].mode == mode; --at) {
+    const Form& f = kForms[at];
     const int T = f.warps;
     TeamKern kern = T == 16 ? team_kern16(mode, multi, var) : T == 8 ? team_kern8(mode, multi, var)
                                                                      : team_kern4(mode, f.blocks, multi, var);
@@ -84,13 +96,13 @@ cudaError_t pick_team(int mode, int s, bool var, bool multi, int64_t nfits, Team
     int wpb = 0, bps = 0;
     e = pick_launch_wpb((const void*)kern, per_warp, T, &wpb, &bps, &sms);
     if (e != cudaSuccess) return e;
-    // Large ROIs: fewer blocks fit an SM than the limits above were taken with. Up to
-    // three waves still win (one warp / team, us: 4Pi 24 px, 300 ROIs, one block per
-    // SM, 1196 / 529, but 600 ROIs 1226 / 1259; 3D 33 px, 800 ROIs 542 / 331).
-    if (n > 3.0 * bps) continue;
     *t = TeamLaunch{kern, 32 * T, per_warp * T};
-    return cudaSuccess;
+    blocks = bps;
+    if (bps >= f.blocks || n <= bps) break;
   }
+  // Several waves win over one warp per ROI up to seven (4Pi, one block per SM, one warp
+  // / team: 7 ROIs per SM 24 px 5,760 / 5,450, 22 px 5,250 / 5,180, but 8 5,250 / 5,820).
+  if (n > kMostWaves * blocks) *t = TeamLaunch{nullptr, 0, 0};
   return cudaSuccess;
 }
 
