@@ -52,17 +52,37 @@ constexpr int64_t kEnoughBatch3D = 12;
 // 4D ROIs, within 0.2% on 200,000 3D ROIs.
 constexpr int64_t kSparePerWarp = 2;
 
-// The most slots with which as many warps stay resident as with one ROI per warp
-// (to 5%), or, where the slots' shared memory leaves none, the most that keep 85% of
-// them (21 px 3D ROIs: 17 warps per SM against 20, and still 1.5% faster). q->slots
-// 0: not even two do. more: floats per warp besides the layout's.
+// The most slots that pay. q->slots 0: not even two do. more: floats per warp besides the
+// layout's. The slots' shared memory costs resident warps or L1, which 3D minds least:
+// - 3D: as many warps as with one ROI per warp (to 5%), else 85% of them (21 px: 17 per SM
+//   against 20, and still 1.5% faster);
+// - 4D: a tenth more warps, which 96 registers allow against 128; with as many, one ROI
+//   per warp is as fast or faster (ms, 60 ROIs per SM: 25 px 4.08 / 4.12, 24 px, 14 warps
+//   against 16, 4.54 / 4.83; 21 px, 18 against 16, 3.04 / 2.97);
+// - 5D: all of the warps, at least 7 (50 ROIs per SM: 25 px, 6 warps, 14.1 / 14.5, 33 px,
+//   4, 27.8 / 29.1; 19 px, 9 against 10, 55 per SM, 8.67 / 9.08), and the gathers' L1:
+//   past the 196 KB configuration of shared memory the SM takes its largest and leaves them
+//   28 KB of 60 (KB of shared memory per SM, ms; 14 px, 36 per SM, one ROI per warp 169,
+//   3.55, three slots 193, 3.50, four 201, 3.97; 15 px, 42 per SM, one ROI per warp 180,
+//   4.41, two slots 195.9, 4.93).
+constexpr int kMinWarps5D = 7;
+constexpr int64_t kSharedL1 = 194 * 1024, kBlockReserve = 1024;  // bytes per SM, per block
+
 cudaError_t most_slots(const void* kern, int mode, int s, bool var, bool multi, int more, int wpb,
                        int64_t warps, SlotLaunch* q) {
-  for (int percent : {95, 85})
+  constexpr int least[3][2] = {{95, 85}, {110, 110}, {100, 100}};  // % of the warps, tried in turn
+  for (int pass = 0; pass < 2; ++pass)
     for (int r = kMaxSlots; r >= 2; --r) {
       SlotLaunch t{r, (make_slot_layout(mode, s, var, r, multi).total + more) * 4, 0, 0, 0};
       if (pick_launch_wpb(kern, t.per_warp, wpb, &t.wpb, &t.bps, &t.sms) != cudaSuccess) continue;
-      if ((int64_t)t.wpb * t.bps * t.sms * 100 < percent * warps) continue;
+      if ((int64_t)t.wpb * t.bps * t.sms * 100 < least[mode - 6][pass] * warps) continue;
+      if (mode == 8) {
+        if (t.wpb * t.bps < kMinWarps5D) continue;
+        const int64_t one = warps / t.sms;  // warps per SM with one ROI each, four per block
+        const int64_t before = one * make_layout(mode, s, var).total() * 4 + (one + 3) / 4 * kBlockReserve;
+        const int64_t now = t.bps * ((int64_t)t.per_warp * t.wpb + kBlockReserve);
+        if (now > kSharedL1 && before <= kSharedL1) continue;
+      }
       *q = t;
       return cudaSuccess;
     }
