@@ -198,14 +198,18 @@ cudaError_t launch_batch(const BatchArgs& a, int mode, bool multi, cudaStream_t 
   BatchKern kern = batch_kern_default(mode, multi, cap);
   if (!kern) return cudaErrorInvalidValue;
   int64_t total = 0;
-  for (int i = 0; i < a.nseg; ++i) total += a.seg[i].n;
+  int segments = 0;
+  for (int i = 0; i < a.nseg; ++i) {
+    total += a.seg[i].n;
+    segments += a.seg[i].n > 0;
+  }
   int per_warp = warp_smem_floats(mode, a.s_max) * 4, rpw = 1;
   int wpb = 4, bps = 0, sms = 0;
   SlotLaunch slots{};
   auto shape = [&](int want) {  // of one ROI per warp, and of the slots that could take its place
     cudaError_t e = pick_launch_wpb((const void*)kern, per_warp, want, &wpb, &bps, &sms);
     if (e == cudaSuccess && !cap)
-      e = pick_slots_batch(mode, a.s_max, multi, total, want, (int64_t)sms * bps * wpb, &slots);
+      e = pick_slots_batch(mode, a.s_max, multi, segments, total, want, (int64_t)sms * bps * wpb, &slots);
     return e;
   };
   cudaError_t e = shape(0);

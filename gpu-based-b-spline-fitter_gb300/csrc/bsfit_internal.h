@@ -227,7 +227,7 @@ struct SlotLaunch {
 };
 cudaError_t pick_slots(int mode, int s, bool var, bool multi, int64_t nfits, int wpb, int64_t warps,
                        SlotLaunch* q);
-cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int64_t total, int wpb, int64_t warps,
+cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int segments, int64_t total, int wpb, int64_t warps,
                              SlotLaunch* q);
 // *taken stays false when the pool has no work counter.
 cudaError_t launch_slots(const FitArgs& a, const SlotLaunch& q, bool* taken, cudaStream_t stream);

@@ -43,10 +43,13 @@ constexpr int64_t kEnough = 3;
 // slots (sized for the largest) are drained at each change. Measured, us, one ROI
 // per warp / slots: 11, 13, 17 px 11,500 ROIs (3.2 W) 380 / 421, 20,000 619 / 657,
 // 36,000 (9.9 W) 1,048 / 1,072, 45,000 (12.3 W) 1,313 / 1,319, 60,000 1,715 / 1,684;
-// 13 px alone 15,000 444 / 457, 20,000 570 / 567, 30,000 806 / 793. 4D 13, 15 px 9,500
-// (3.9 W) 1,891 / 1,876, 20,000 3,655 / 3,575; 5D 17 px 5,600 5,041 / 5,035, 14,000
-// 11,671 / 11,548.
-constexpr int64_t kEnoughBatch3D = 12;
+// 13 px alone 15,000 444 / 457, 20,000 570 / 567, 30,000 806 / 793. A 4D or 5D batch of
+// one segment does as its plain call (4D 13 px 4 W 1,752 / 1,699, 5D 13 px 3.1 W 3,219 /
+// 3,242, 4 W 4,057 / 3,952), but several lose at each change until their number is small
+// against the work: 4D 13, 15 px, two segments 4 W 1,893 / 1,914, 6 W 2,724 / 2,839, 8 W
+// 3,558 / 3,528, four 5 W 2,320 / 2,630, 8 W 3,551 / 3,349; 5D 13 px, two 5 W 4,957 /
+// 5,667, 6 W 5,866 / 6,371, 8 W 7,659 / 7,655, 12 W 11,236 / 10,587.
+constexpr int64_t kEnoughBatch3D = 12, kEnoughSegments = 8;
 // Warps stop taking further ROIs when two per warp are left: 0, 1, 2, 3 measured
 // 7.54, 7.01, 6.68, 6.77 ms on 8,000 5D ROIs, 5.68, 5.64, 5.54, 5.60 ms on 40,000
 // 4D ROIs, within 0.2% on 200,000 3D ROIs.
@@ -99,10 +102,10 @@ cudaError_t pick_slots(int mode, int s, bool var, bool multi, int64_t nfits, int
   return kern ? most_slots((const void*)kern, mode, s, var, multi, 0, wpb, warps, q) : cudaSuccess;
 }
 
-cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int64_t total, int wpb, int64_t warps,
+cudaError_t pick_slots_batch(int mode, int s_max, bool multi, int segments, int64_t total, int wpb, int64_t warps,
                              SlotLaunch* q) {
   *q = SlotLaunch{};
-  if (total < (mode == 6 ? kEnoughBatch3D : kEnough) * warps) return cudaSuccess;
+  if (total < (mode == 6 ? kEnoughBatch3D : segments > 1 ? kEnoughSegments : kEnough) * warps) return cudaSuccess;
   const BatchKern kern = slot_batch_kern(mode, multi);
   return kern ? most_slots((const void*)kern, mode, s_max, false, multi, kSegWords, wpb, warps, q) : cudaSuccess;
 }

@@ -31,3 +31,26 @@ def test_place(bsfit_mod, fittype, s, slots):
     names = captured(lambda: m.fit_torch(lots, 5))[1]
     assert any("slot_kernel" in k for k in names) == slots, names
     m.close()
+
+
+@pytest.mark.parametrize("fittype,per_sm,segments,slots", [
+    (7, 56, 1, True), (7, 80, 2, False), (7, 80, 4, False), (7, 140, 2, True), (8, 42, 1, True), (8, 60, 2, False),
+    (8, 110, 3, True), (6, 120, 2, False), (6, 320, 2, True)])
+def test_batches_by_segments(bsfit_mod, fittype, per_sm, segments, slots):
+    import torch
+    from bsfit import workloads as W
+    few, n = 30, 152 * per_sm // segments
+    w = (W.workload_3d(few, s=13, stream=991) if fittype == 6 else
+         W.workload_4d(few, sizes=(13,), stream=992)[0] if fittype == 7 else W.workload_5d(few, s=13, stream=993))
+    m = bsfit_mod.Model(fittype, w.coeff, coeff3=w.coeff3, init_p=w.init_p)
+    idx = np.random.default_rng(9).integers(0, few, n)
+    r = torch.from_numpy(w.rois).cuda()
+    lots = r[torch.from_numpy(idx).cuda()].contiguous()
+    b = bsfit_mod.Batch([(m, lots, 4)] * segments)
+    ref = m.fit_torch(r, 4)
+    for out in b.run():
+        for x, y in zip(out, ref):
+            assert np.array_equal(x.cpu().numpy(), np.take(y.cpu().numpy(), idx, axis=-1), equal_nan=True)
+    names = captured(lambda: b.run())[1]
+    assert any("slot_batch_kernel" in k for k in names) == slots, names
+    m.close()
