@@ -1365,7 +1365,7 @@ template <int MODE>
 constexpr int kMaxWarps = MODE == 6 ? 16 : MODE == 7 ? 12 : 8;
 
 template <int MODE, bool STEP>
-__global__ void __launch_bounds__(STEP ? 32 * kMaxWarps<MODE> : 128, STEP ? 1 : 4) fitdd_kernel(FitArgs a) {
+__global__ void __launch_bounds__(STEP ? 32 * kMaxWarps<MODE> : 128, STEP || MODE != 6 ? 1 : 4) fitdd_kernel(FitArgs a) {
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   constexpr int NV = Traits<MODE>::NV;
@@ -1448,8 +1448,29 @@ __global__ void __launch_bounds__(128) evaldd_kernel(FitArgs a, const float* the
 }  // namespace ddf
 
 constexpr int kMaxShared = 227 * 1024;  // bytes per block
-constexpr int kAlone3D = 7;             // most ROIs per SM of a 3D call fitted on their own
 constexpr int kInStep3D = 8;            // fewest warps per SM for 3D fits in step
+
+// Whether a call's fits run on their own, in small blocks, instead of in step: few warps
+// compete for the instruction cache, and in step they wait for the slowest. Measured, us
+// (on their own / in step):
+// - 3D up to 8 ROIs per SM: 7 ROIs 5 px 283 / 310, 7 px 326 / 353, 13 px 319 / 328, 21 px 611 /
+//   633; 8 7 px 327 / 372, 15 px 409 / 411, 19 px 566 / 535, 21 px 609 / 652. ROIs of up to
+//   9 px, whose evaluations are short, up to 9.5: 9 ROIs 5 px 328 / 337, 7 px 370 / 385, 9 px
+//   313 / 309 (another sample 361 / 408); 10 5 px 347 / 345, 7 px 389 / 386; 13 px 9 396 / 386.
+// - 3D where shared memory holds fewer than eight warps per SM (4,000 ROIs, four iterations:
+//   23 px, 7 warps, 992 / 1,002, 27 px, 6 warps, 1,520 / 1,774).
+// - 4D up to 4 ROIs per SM (1 ROI 9 px 887 / 915, 13 px 1,237 / 1,316, 4 17 px 1,786 / 1,834;
+//   4.3 13 px 1,611 / 1,628, 17 px 2,335 / 2,381, but 5.6 13 px 1,717 / 1,668).
+// - 5D of 17 px and more, from more than 1 to 3 (17 px 1.4 ROIs 5,303 / 5,481, 2 5,291 / 5,516,
+//   3 5,437 / 5,540, 3.5 5,634 / 5,478; 1 ROI 5,291 / 5,176, where blocks of four leave SMs
+//   without a ROI; 13 px 1.4 3,606 / 3,572, 2 3,617 / 3,668, 3 3,718 / 3,716).
+// From 8 to 10 ROIs per SM 3D calls differ by up to 5% either way with the sample.
+static bool alone(int mode, int s, int64_t nfits, int sms, int most) {
+  const double n = (double)nfits / sms;
+  if (mode == 6) return most < kInStep3D || n <= 8.0 || (s <= 9 && n <= 9.5);
+  if (mode == 7) return n <= 4.0;
+  return s >= 17 && n > 1.0 && n <= 3.0;
+}
 
 int fitdd_smem_floats(int mode, int s) { return ddf::make_layout(mode, s).total(); }
 
@@ -1476,11 +1497,11 @@ cudaError_t launch_evaldd(const FitArgs& a, const float* theta, double* out, int
 cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream) {
   if (a.nfits <= 0) return cudaSuccess;
   const int mode = a.m.fittype;
-  void (*kern)(FitArgs) = nullptr;
+  FitKern kern = nullptr, own = nullptr;
   int most = 0;
-  if (mode == 6) kern = ddf::fitdd_kernel<6, true>, most = ddf::kMaxWarps<6>;
-  else if (mode == 7) kern = ddf::fitdd_kernel<7, true>, most = ddf::kMaxWarps<7>;
-  else if (mode == 8) kern = ddf::fitdd_kernel<8, true>, most = ddf::kMaxWarps<8>;
+  if (mode == 6) kern = ddf::fitdd_kernel<6, true>, own = ddf::fitdd_kernel<6, false>, most = ddf::kMaxWarps<6>;
+  else if (mode == 7) kern = ddf::fitdd_kernel<7, true>, own = ddf::fitdd_kernel<7, false>, most = ddf::kMaxWarps<7>;
+  else if (mode == 8) kern = ddf::fitdd_kernel<8, true>, own = ddf::fitdd_kernel<8, false>, most = ddf::kMaxWarps<8>;
   else return cudaErrorInvalidValue;
   const int per_warp = (fitdd_smem_floats(mode, a.s) * 4 + 15) & ~15;
   int dev = 0, sms = 0;
@@ -1488,22 +1509,17 @@ cudaError_t launch_fitdd(const FitArgs& a, cudaStream_t stream) {
   if (e == cudaSuccess) e = sm_count(dev, &sms);
   if (e != cudaSuccess) return e;
   if (most > kMaxShared / per_warp) most = kMaxShared / per_warp;
-  // 3D fits that leave the SMs nearly empty, or of which few fit an SM's shared memory,
-  // run on their own in small blocks: few warps compete for the instruction cache, and
-  // in step they wait for the slowest (us, in step / on their own; 7 px: 600 ROIs
-  // 317 / 298, 1,000 376 / 311, 1,700 407 / 403; 13 px: 285 / 272, 336 / 318,
-  // 407 / 430; 21 px, 1,300 ROIs 688 / 829; 4,000 ROIs, four iterations: 23 px, 7 warps
-  // per SM, 1,002 / 992, 27 px, 6 warps, 1,774 / 1,520). For 4D and 5D in step is as
-  // fast or faster from the start (5D, 800 ROIs 5,301 / 6,669).
   int wpb = 4, bps = 0;
-  if (mode == 6 && (most < kInStep3D || a.nfits <= (int64_t)kAlone3D * sms)) {
-    kern = ddf::fitdd_kernel<6, false>;
+  if (alone(mode, a.s, a.nfits, sms, most)) {
+    kern = own;
     e = pick_launch((const void*)kern, per_warp, &wpb, &bps, &sms);
   } else {
-    // Whole quads, so that every scheduler has the same number of warps (10,000 ROIs:
-    // 3D 21 px 9 warps 3,691 us, 8 warps 3,428; 5D 17 px 7 warps 82,100, 4 77,900).
-    if (most > 4) most &= ~3;
+    // One wave if the warps hold the call (19 px, 10 ROIs per SM, 10 warps 642 us, 8 and a
+    // second wave 861), else whole quads, so that every scheduler has the same number
+    // (10,000 ROIs: 3D 21 px 9 warps 3,691 us, 8 warps 3,428; 5D 17 px 7 warps 82,100, 4
+    // 77,900).
     const int64_t each = (a.nfits + sms - 1) / sms;
+    if (each > most && most > 4) most &= ~3;
     wpb = each < most ? (int)each : most < 1 ? 1 : most;
     e = pick_launch_wpb((const void*)kern, per_warp, wpb, &wpb, &bps, &sms);
   }

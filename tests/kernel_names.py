@@ -10,9 +10,9 @@ class _KernelParams(ctypes.Structure):  # CUDA_KERNEL_NODE_PARAMS
                 ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
 
 
-def captured(call):
-    """(node types, names of the kernels as the linker knows them) of ``call()``, captured on a
-    stream of its own and not run."""
+def launches(call):
+    """[(node type, kernel name as the linker knows it, blocks, threads per block)] of
+    ``call()``, captured on a stream of its own and not run (name None: not a kernel)."""
     import torch
     cu = ctypes.CDLL("libcuda.so.1")
     graph = torch.cuda.CUDAGraph(keep_graph=True)
@@ -23,15 +23,22 @@ def captured(call):
     assert cu.cuGraphGetNodes(raw, None, ctypes.byref(count)) == 0
     nodes = (ctypes.c_void_p * count.value)()
     assert cu.cuGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
-    types, names = [], []
+    found = []
     for n in nodes:
         t = ctypes.c_int()
         assert cu.cuGraphNodeGetType(ctypes.c_void_p(n), ctypes.byref(t)) == 0
-        types.append(t.value)
-        if t.value == KERNEL:
-            p, name = _KernelParams(), ctypes.c_char_p()
-            assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(n), ctypes.byref(p)) == 0
-            get = (cu.cuKernelGetName, p.kern) if p.kern else (cu.cuFuncGetName, p.func)
-            assert get[0](ctypes.byref(name), ctypes.c_void_p(get[1])) == 0
-            names.append(name.value.decode())
-    return types, names
+        if t.value != KERNEL:
+            found.append((t.value, None, 0, 0))
+            continue
+        p, name = _KernelParams(), ctypes.c_char_p()
+        assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(n), ctypes.byref(p)) == 0
+        get = (cu.cuKernelGetName, p.kern) if p.kern else (cu.cuFuncGetName, p.func)
+        assert get[0](ctypes.byref(name), ctypes.c_void_p(get[1])) == 0
+        found.append((KERNEL, name.value.decode(), p.grid[0], p.block[0]))
+    return found
+
+
+def captured(call):
+    """(node types, kernel names) of ``call()``."""
+    found = launches(call)
+    return [f[0] for f in found], [f[1] for f in found if f[1]]
