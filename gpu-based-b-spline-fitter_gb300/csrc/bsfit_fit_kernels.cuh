@@ -1085,54 +1085,6 @@ __device__ void evaluate(const FitArgs& a, const WarpLayout& L, float* ws, int l
 }
 
 // ---------------------------------------------------------------------------
-// LM helpers (warp-uniform register state).
-
-
-// Unpivoted Cholesky of the full matrix a (row-major NV x NV), lower factor in
-// u (u[i*NV + j], j <= i). Fails on a negative pivot only
-// (CPUsplineLib.cpp:1363-1390).
-template <int NV>
-__device__ __forceinline__ bool cholesky(const float (&a)[NV * NV], float (&u)[NV * NV]) {
-#pragma unroll
-  for (int i = 0; i < NV; i++) {
-#pragma unroll
-    for (int j = 0; j <= i; j++) {
-      float s = 0.0f;
-#pragma unroll
-      for (int k = 0; k < j; k++) s = fmaf(u[i * NV + k], u[j * NV + k], s);
-      if (i == j) {
-        float piv = a[i * NV + i] - s;
-        if (!(piv >= 0.0f)) return false;
-        u[i * NV + j] = sqrtf(piv);
-      } else {
-        u[i * NV + j] = (a[i * NV + j] - s) / u[j * NV + j];
-      }
-    }
-  }
-  return true;
-}
-
-template <int NV>
-__device__ __forceinline__ void chol_solve(const float (&u)[NV * NV], const float (&b)[NV],
-                                           float (&x)[NV]) {
-  float y[NV];
-#pragma unroll
-  for (int i = 0; i < NV; i++) {
-    float t = b[i];
-#pragma unroll
-    for (int j = 0; j < i; j++) t -= u[i * NV + j] * y[j];
-    y[i] = t / u[i * NV + i];
-  }
-#pragma unroll
-  for (int i = NV - 1; i >= 0; i--) {
-    float t = y[i];
-#pragma unroll
-    for (int j = i + 1; j < NV; j++) t -= u[j * NV + i] * x[j];
-    x[i] = t / u[i * NV + i];
-  }
-}
-
-// ---------------------------------------------------------------------------
 // One ROI, one warp. The LM state is distributed over the lanes: lane l < NV
 // owns parameter l (value, previous value, sign, clamp), gradient entry l and
 // Hessian row l, so the small dense algebra of each step runs lane-parallel
