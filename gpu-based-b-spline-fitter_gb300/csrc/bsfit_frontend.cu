@@ -89,7 +89,7 @@ __global__ void prepare_frames(FrontArgs a) {
 // is above the cutoff. Keeping the filtered tile on chip leaves one read of the
 // frames. 64 frames of 512 x 512, 7 x 7 kernel: 73 us (92 us with scalar FMAs)
 // against 282 us for a filter with its sums in rows and 143 us for a counting and
-// a writing pass over the filtered image; the whole call 600 -> 177 us.
+// a writing pass over the filtered image; the whole call 605 -> 195 us.
 template <int K>
 __global__ void __launch_bounds__(32 * kGroups)
     filter_maxima(const __grid_constant__ FrontArgs a, const __grid_constant__ Filter flt) {

@@ -236,7 +236,7 @@ cudaError_t launch_slots_batch(const BatchArgs& a, int mode, bool multi, const S
 // most warps resident; blocks per SM; SM count), cached per kernel, size and
 // device.
 cudaError_t pick_launch(const void* kern, int per_warp, int* wpb, int* bps, int* sms);
-// The same with the warps per block forced (force_wpb a power of two; 0 chooses).
+// The same with the warps per block forced (force_wpb any number; 0 chooses).
 cudaError_t pick_launch_wpb(const void* kern, int per_warp, int force_wpb, int* wpb, int* bps,
                             int* sms);
 
