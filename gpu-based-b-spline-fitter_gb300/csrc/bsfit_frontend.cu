@@ -239,16 +239,25 @@ __global__ void scan_counts(const int* counts, long long* offsets, int64_t n) {
 }
 
 // Coordinates and cut-outs of one tile column's maxima (kTX columns of a frame),
-// one block each: the mask words in scan order (columns, then rows) are counted
-// per thread and prefix-summed over the block, every thread writes its maxima's
-// coordinates, then the warps cut the ROIs out.
-__global__ void __launch_bounds__(256) write_rois(const __grid_constant__ FrontArgs a) {
+// blockIdx.y's share of them: the mask words in scan order (columns, then rows) are
+// counted per thread and prefix-summed over the block, every thread writes the
+// coordinates of its maxima in the share, then the warps cut the ROIs out.
+//
+// The shares fill the GPU where a movie has few tile columns: with one block per column
+// the cut-out of a frame of many maxima is the work of 18 or 69 blocks (us per call,
+// without / with shares: 512 x 512, 7 x 7 kernel, 23,700 maxima 210 / 110, 2048 x 2048,
+// 254,000 690 / 241; 369 in 512 x 512 91 / 93, 64 frames with 24,000 168 / 170).
+constexpr int kCutThreads = 256;
+__global__ void __launch_bounds__(kCutThreads) write_rois(const __grid_constant__ FrontArgs a) {
   __shared__ int part[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t f = blockIdx.x / a.xtiles;
   const int xt = (int)(blockIdx.x - f * a.xtiles);
   const long long base = a.offsets[blockIdx.x], end = a.offsets[blockIdx.x + 1];
-  if (base == end || base >= a.capacity) return;
+  int share = (int)((unsigned)(end - base) + gridDim.y - 1) / (int)gridDim.y;
+  if (share < kCutThreads >> 5) share = kCutThreads >> 5;  // a ROI per warp at least
+  const long long k0 = base + (long long)share * blockIdx.y, k1 = k0 + share < end ? k0 + share : end;
+  if (k0 >= k1 || k0 >= a.capacity) return;
   const int64_t xb = (int64_t)xt * kTX;
   const int cols = (int)(a.W - xb < kTX ? a.W - xb : kTX);
   const int64_t words = (int64_t)cols * a.ytiles * 2;
@@ -272,7 +281,7 @@ __global__ void __launch_bounds__(256) write_rois(const __grid_constant__ FrontA
     while (m) {
       const int r = __ffs(m) - 1;
       m &= m - 1;
-      if (idx < a.capacity) {
+      if (idx >= k0 && idx < k1 && idx < a.capacity) {
         a.coords[idx] = (float)(xb + column + 1);
         a.coords[a.capacity + idx] = (float)((q >> 1) * kTY - 1 + (q & 1) * 32 + r + 1);
         a.coords[2 * a.capacity + idx] = (float)(f + 1);
@@ -281,9 +290,9 @@ __global__ void __launch_bounds__(256) write_rois(const __grid_constant__ FrontA
     }
   }
   __syncthreads();
-  const long long n = end < a.capacity ? end : a.capacity;
+  const long long n = k1 < a.capacity ? k1 : a.capacity;
   const int s = a.s, s2 = s * s, dx = a.dx;
-  for (long long k = base + warp; k < n; k += blockDim.x >> 5) {
+  for (long long k = k0 + warp; k < n; k += blockDim.x >> 5) {
     const int64_t cx = (int64_t)a.coords[k] - 1, cy = (int64_t)a.coords[a.capacity + k] - 1;
     float* roi = a.rois + k * s2;
     for (int p = lane; p < s2; p += 32) {
@@ -429,8 +438,17 @@ int bsfit_find_rois_device(const float* d_frames, int64_t nframes, int64_t heigh
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && capacity > 0) {
-    bsfit::write_rois<<<(unsigned)tcols, 256, 0, st>>>(a);
-    e = cudaGetLastError();
+    // no more blocks than are resident, eight on an SM: a second wave costs more than it
+    // evens out (64 frames of 512 x 512, one / two shares 160 / 170 us); 16 shares leave a
+    // warp few ROIs already
+    int dev = 0, sms = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = bsfit::sm_count(dev, &sms);
+    if (e == cudaSuccess) {
+      const int64_t fit = 8 * (int64_t)sms / tcols, shares = fit < 1 ? 1 : fit < 16 ? fit : 16;
+      bsfit::write_rois<<<dim3((unsigned)tcols, (unsigned)shares), bsfit::kCutThreads, 0, st>>>(a);
+      e = cudaGetLastError();
+    }
   }
   long long total = 0;
   if (e == cudaSuccess)
