@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <utility>
 
 #include "../../include/bsfit.h"
 #include "bsfit_internal.h"
@@ -84,9 +85,11 @@ __global__ void prepare_frames(FrontArgs a) {
 // The filter is bound by its multiply-adds (49 per pixel for a 7 x 7 kernel):
 // each thread takes rows r and r + 32 in the halves of paired FMAs and kCols
 // neighbouring columns, reads a column's k row pairs into registers once for all
-// of them (k (kCols + k - 1) shared loads for kCols k^2 paired FMAs), and K > 0
-// unrolls the sum (K = 0: any size). A pixel's neighbours are only read where it
-// is above the cutoff. Keeping the filtered tile on chip leaves one read of the
+// of them (k (kCols + k - 1) shared loads for kCols k^2 paired FMAs), for which the
+// size has to be known: a loop over any size, its columns read again for every term, took
+// up to twice the time of a call (us, loop / this: 31 x 31 kernel, 30 frames of 100 x 100
+// 200 / 106, 64 of 512 x 512 2,190 / 1,240; 14 x 14, 64 of 512 x 512 513 / 287). A pixel's
+// neighbours are only read where it is above the cutoff. Keeping the filtered tile on chip leaves one read of the
 // frames. 64 frames of 512 x 512, 7 x 7 kernel: 73 us (92 us with scalar FMAs)
 // against 282 us for a filter with its sums in rows and 143 us for a counting and
 // a writing pass over the filtered image; the whole call 605 -> 195 us.
@@ -95,8 +98,8 @@ __global__ void __launch_bounds__(32 * kGroups)
     filter_maxima(const __grid_constant__ FrontArgs a, const __grid_constant__ Filter flt) {
   extern __shared__ float2 tile2[];  // [kFX + k - 1][32 + k - 1]: rows q and q + 32
   float* tile = reinterpret_cast<float*>(tile2);  // then the filtered [kFX][kFY]
-  const int k = K > 0 ? K : a.k, o = (k - 1) / 2;
-  const int ty = kFY + k - 1, tx = kFX + k - 1, py = 32 + k - 1;
+  constexpr int k = K, o = (k - 1) / 2;
+  constexpr int ty = kFY + k - 1, tx = kFX + k - 1, py = 32 + k - 1;
   const int64_t f = blockIdx.z;
   const int64_t y0 = (int64_t)blockIdx.x * kTY - 1, x0 = (int64_t)blockIdx.y * kTX - 1;
   const int row = threadIdx.x, grp = threadIdx.y;
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(32 * kGroups)
       if (twice) d[32].x = vb;
     }
     for (int i = grp * 32 + row; i < (k - 1) * tx; i += 32 * kGroups) {
-      const int cx = i / (k - 1), e = i - cx * (k - 1);
+      const int cx = i / (k > 1 ? k - 1 : 1), e = i - cx * (k - 1);
       float v = 0.0f;
       if (cx >= cx0 && cx < cx1 && kFY + e < cy1) v = pixel(img + cx * a.H + kFY + e);
       tile2[cx * py + 32 + e].y = v;
@@ -136,26 +139,19 @@ __global__ void __launch_bounds__(32 * kGroups)
 #pragma unroll
   for (int i = 0; i < kCols; ++i) acc[i] = make_float2(0.0f, 0.0f);
   const float2* col = tile2 + grp * kCols * py + row;
-  if constexpr (K > 0) {
 #pragma unroll
-    for (int c = 0; c < kCols + K - 1; ++c) {
-      float2 x[K];
+  for (int c = 0; c < kCols + k - 1; ++c) {
+    float2 x[k];
 #pragma unroll
-      for (int u = 0; u < K; ++u) x[u] = col[c * py + u];
+    for (int u = 0; u < k; ++u) x[u] = col[c * py + u];
 #pragma unroll
-      for (int i = 0; i < kCols; ++i) {
-        const int v = c - i;
-        if (v >= 0 && v < K) {
+    for (int i = 0; i < kCols; ++i) {
+      const int v = c - i;
+      if (v >= 0 && v < k) {
 #pragma unroll
-          for (int u = 0; u < K; ++u) acc[i] = __ffma2_rn(flt.h[u + K * v], x[u], acc[i]);
-        }
+        for (int u = 0; u < k; ++u) acc[i] = __ffma2_rn(flt.h[u + k * v], x[u], acc[i]);
       }
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kCols; ++i)
-      for (int v = 0; v < k; ++v)
-        for (int u = 0; u < k; ++u) acc[i] = __ffma2_rn(flt.h[u + k * v], col[(i + v) * py + u], acc[i]);
   }
   __syncthreads();  // the tile is read; the filtered one goes over it
 #pragma unroll
@@ -305,24 +301,14 @@ __global__ void __launch_bounds__(kCutThreads) write_rois(const __grid_constant_
 
 using FilterKern = void (*)(const FrontArgs, const Filter);
 
-// Kernel sizes unrolled: differences of Gaussians of sigma 0.3 to 2 and Gaussians
-// to sigma 4 have 3 to 13; the others run the loop form.
-FilterKern filter_kern(int k) {
-  switch (k) {
-    case 3: return filter_maxima<3>;
-    case 4: return filter_maxima<4>;
-    case 5: return filter_maxima<5>;
-    case 6: return filter_maxima<6>;
-    case 7: return filter_maxima<7>;
-    case 8: return filter_maxima<8>;
-    case 9: return filter_maxima<9>;
-    case 10: return filter_maxima<10>;
-    case 11: return filter_maxima<11>;
-    case 12: return filter_maxima<12>;
-    case 13: return filter_maxima<13>;
-    default: return filter_maxima<0>;
-  }
+template <int... I>
+FilterKern filter_kern_of(int k, std::integer_sequence<int, I...>) {
+  constexpr FilterKern kern[] = {filter_maxima<I + 1>...};
+  return kern[k - 1];
 }
+
+// The kernel of a filter size, 1 to kMaxKernel.
+FilterKern filter_kern(int k) { return filter_kern_of(k, std::make_integer_sequence<int, kMaxKernel>()); }
 
 }  // namespace
 }  // namespace bsfit
