@@ -182,6 +182,8 @@ struct ModeTraits<8> {
 // model's 10 maps (GP = 10: a half-warp's sixteen consecutive items sit 10
 // banks apart, 2 banks each, all distinct), and otherwise with GP odd (the
 // consecutive items of a pass an odd stride apart: 32 distinct banks).
+constexpr int kBestFloats = 16;
+
 struct WarpLayout {
   int s, s2p, wp, na, ng, nch, nvar;  // nvar: sCMOS variance planes (0 or nch)
   bool alias;
@@ -200,7 +202,9 @@ struct WarpLayout {
   __host__ __device__ constexpr int off_ky() const { return off_kx() + ((s + 3) & ~3); }
   __host__ __device__ constexpr int off_w() const { return off_ky() + ((s + 3) & ~3); }
   __host__ __device__ constexpr int off_dt() const { return off_w() + 40; }
-  __host__ __device__ constexpr int off_maps() const { return off_dt() + (nch > 1 ? nch * 6 : 0); }
+  // 4Pi: the kept result of several starts (fit_and_store)
+  __host__ __device__ constexpr int off_best() const { return off_dt() + (nch > 1 ? nch * 6 : 0); }
+  __host__ __device__ constexpr int off_maps() const { return off_best() + (nch > 1 ? kBestFloats : 0); }
   __host__ __device__ constexpr int a_rel() const {
     return alias ? gs() + (wp - 1) * (gs() > as() ? gs() - as() : 0) : wp * gs();
   }
@@ -246,7 +250,7 @@ constexpr bool layouts_disjoint() {
         const WarpLayout L = make_layout(modes[mi], s, var != 0);
         if ((L.nch + L.nvar) * s * s > L.off_kx() || L.off_kx() + s > L.off_ky() ||
             L.off_ky() + s > L.off_w() || L.off_w() + 5 * 8 > L.off_dt() ||
-            L.off_dt() + (L.nch > 1 ? L.nch * 6 : 0) > L.off_maps() ||
+            L.off_dt() + (L.nch > 1 ? L.nch * 6 + 14 : 0) > L.off_maps() ||
             L.off_a() + L.wp * L.as() > L.total() || L.off_g() + L.wp * L.gs() > L.total())
           return false;
         for (int c = 0; c < L.wp; ++c)
@@ -1719,10 +1723,35 @@ __device__ __forceinline__ void fit_and_store(const FitArgs& a, const WarpLayout
     // double the kernel's instruction footprint)
     RoiResult best{0.0f, 0.0f, 0.0f, 0};
     const int ns = a.n_starts > 0 ? a.n_starts : 1;  // 0: the model's initP alone
+    // 4Pi keeps the better result in shared memory (par and crlb of six lanes, ll, kk):
+    // four more registers through the fits had the evaluation spill (us, 1,500 ROIs of
+    // 12 px, two starts: in registers 5,680, in shared memory 4,870).
+    constexpr bool kShared = ModeTraits<MODE>::NCH > 1;
+    constexpr int NV = ModeTraits<MODE>::NV;
+    static_assert(!kShared || 2 * NV + 2 <= kBestFloats, "room of the kept result");
+    float* kept = ws + L.off_best();
     for (int k = 0; k < ns; ++k) {
       const RoiResult r = fit_roi<MODE>(a, L, ws, lane, roi, k);
-      const float d = r.ll - best.ll;
-      if (k == 0 || (a.strict ? (d > 1e-4f) : (d >= 1e-4f))) best = r;
+      const float d = r.ll - (kShared && k > 0 ? kept[2 * NV] : best.ll);
+      const bool better = k == 0 || (a.strict ? (d > 1e-4f) : (d >= 1e-4f));
+      if constexpr (kShared) {
+        __syncwarp();
+        if (better && lane < NV) {
+          kept[lane] = r.par;
+          kept[NV + lane] = r.crlb;
+        }
+        if (better && lane == 0) {
+          kept[2 * NV] = r.ll;
+          kept[2 * NV + 1] = __int_as_float(r.kk);
+        }
+        __syncwarp();
+      } else if (better) {
+        best = r;
+      }
+    }
+    if constexpr (kShared) {
+      const int i = lane < NV ? lane : 0;
+      best = RoiResult{kept[i], kept[NV + i], kept[2 * NV], __float_as_int(kept[2 * NV + 1])};
     }
     store_result<MODE>(a, lane, roi, best);
   } else {
